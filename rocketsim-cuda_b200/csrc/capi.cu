@@ -24,7 +24,7 @@ RSX_DECL_PERSIST(16)
 #define RSX_DECL_LOCKSTEP(T)                                                                                                \
   cudaError_t rsx_launch_sim8_lockstep_t##T(uint32_t* states, const void* sds, const uint8_t* sd_index, const void* controls,         \
                                             uint32_t* result, uint32_t* ev_or, const uint32_t* order, uint32_t* counter, uint32_t n,  \
-                                            uint32_t grid, uint32_t block, int split, uint32_t t_first, uint32_t t_last,                \
+                                            uint32_t width, uint32_t grid, uint32_t block, int split, uint32_t t_first, uint32_t t_last, \
                                             cudaStream_t s);
 RSX_DECL_LOCKSTEP(448)
 RSX_DECL_LOCKSTEP(512)
@@ -301,11 +301,11 @@ int rsx_sim8_lockstep_ex(uint32_t* d_states, uint32_t n, const void* d_statics, 
     RSX_CK(cudaMemsetAsync(d_queue_counter, 0, 4, s));
     cudaError_t e;
     if (block <= 448)
-      e = rsx_launch_sim8_lockstep_t448(d_states, d_statics, d_sd_index, d_controls, d_result, d_event_or, d_order, d_queue_counter, n, grid,
-                                        block, (int)split, t0, t1, s);
+      e = rsx_launch_sim8_lockstep_t448(d_states, d_statics, d_sd_index, d_controls, d_result, d_event_or, d_order, d_queue_counter, n, 32,
+                                        grid, block, (int)split, t0, t1, s);
     else
-      e = rsx_launch_sim8_lockstep_t512(d_states, d_statics, d_sd_index, d_controls, d_result, d_event_or, d_order, d_queue_counter, n, grid,
-                                        block, (int)split, t0, t1, s);
+      e = rsx_launch_sim8_lockstep_t512(d_states, d_statics, d_sd_index, d_controls, d_result, d_event_or, d_order, d_queue_counter, n, 32,
+                                        grid, block, (int)split, t0, t1, s);
     RSX_CK(e);
   }
   return RSX_OK;

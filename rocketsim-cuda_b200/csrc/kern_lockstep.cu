@@ -12,23 +12,26 @@
 // the barriers out between P3b (4) or P4 (5) and P8, to measure what they buy), so that at any time the block's warps
 // fetch from one piece of code.  Splits 9 and 10 add the pooled contact work below; split 11 is split 10 with P3a in
 // one piece again (once P3b and the rays were pooled, P3a's per-body barriers cost more than they kept together);
-// split 14 is split 11 with the box-triangle SATs' feature pairs computed by the whole block; split 15 is split 14 with
-// the wheel rays' mesh walks run by the whole block level by level.
+// split 14 is split 11 with the box-triangle SATs' feature pairs computed by the whole block; split 15 runs all of a
+// tick's mesh work (the wheel rays of both cars, every mesh pair of P3b) in one round each, its BVH walks too by the whole
+// block, level by level.
 //
 // Work: `gridDim.x` resident blocks (normally one per SM, `blockDim.x` up to RSX_LS_MAXT threads); every warp claims
-// 32 consecutive entries of `order` (arena indices; identity when null) with one atomicAdd on `counter` (zero at
-// launch) whenever its previous 32 arenas have finished this launch's ticks (t_first..t_last of the decision's 8), and
-// loads them at the next tick boundary.  A decision split over several launches carries each arena's progress in its
-// result word (scored tick, unimplemented bit) and event word; an arena scored in an earlier launch is not stepped
-// again.  The
-// block leaves when no warp holds work.  Lanes past n (and order entries past n) step a copy of an arena and store nothing.
+// `width` (up to 32) consecutive entries of `order` (arena indices; identity when null) whenever its previous arenas have
+// finished this launch's ticks (t_first..t_last of the decision's 8), with one atomicAdd on `counter` (zero at launch) or,
+// when counter is null, its own share of the entries in turn, and loads them at the next tick boundary.  A claim narrower
+// than a warp leaves its other lanes without an arena; they still take part in the block's pooled work.  A decision split
+// over several launches carries each arena's progress in its result word (scored tick, unimplemented bit) and event
+// word; an arena scored in an earlier launch is not stepped again.  The block leaves when no warp holds work.  Lanes past
+// n (and order entries past n) step nothing.
 //
 // Results: each arena's decision is the decide() sequence of sim/physics.cuh (controls before every tick, all 8 ticks
 // stepped, the state after the first scored tick kept, event OR up to that tick), so states, result words and event
 // words equal those of every other decision kernel, whatever grid, block, split or order.
 //
-// Compiled once per register budget (RSX_LS_MAXT threads per block, one block per SM: 448 -> 144 registers,
-// 512 -> 128).
+// Compiled once per register budget (RSX_LS_MAXT threads per block, one block per SM; a scheduler holds a quarter of the
+// registers and of the warps): 256 threads -> 255 registers, 384 -> 168, 448 and 512 -> 128.  The first two hold split 15
+// only (RSX_LS_WIDE_REGS).
 #include "kern_common.cuh"
 
 #ifndef RSX_LS_MAXT
@@ -93,38 +96,80 @@ struct RayPoolSmem {
   uint32_t pair_leaf[kRayPairs];
   sim::RayLeaf out[kRayPairs];
 };
-// split 15: the wheel rays' mesh walks pooled too.  The block walks every mesh job's BVHs level by level (front: the
-// nodes of one level, each a slot | mesh << 6 | node << 10 and its path key); leaves go to a list (slot | mesh << 6 |
-// leaf << 10, key), a counting sort by slot and an insertion sort by key within each slot give every job its leaves in
-// the stack walk's order (sim/ray.cuh walk_expand).  Any list past its capacity sends the round to the serial walks.
-constexpr int kRayFront = 256;
-struct RayWalkSmem {
-  sim::RayMeshJob job[kRayJobs];
-  const StaticData* jd[kRayJobs];
-  Box3 jbox[kRayJobs];
-  uint32_t jbody[kRayJobs];
-  uint32_t cnt[kRayJobs], seg[kRayJobs], fill[kRayJobs];
-  uint32_t leaf_a[kRayPairs], key_a[kRayPairs];  // as found
-  uint32_t leaf_b[kRayPairs], key_b[kRayPairs];  // by slot, then by key
-  sim::RayLeaf out[kRayPairs];
-  uint32_t front[2][kRayFront][2];
-  uint32_t nfront[sim::kWalkLevels + 1], nleaf, ovf;
+// split 15: mesh walks by the whole block.  Jobs (a body's query box against a mesh body) are listed in shared memory,
+// the block walks all their BVHs level by level (front: the nodes of one level with their path keys, sim/ray.cuh
+// walk_expand), and the leaves found are put in each job's stack-walk order by a counting sort by job and a ranking by
+// key within the job.  A job that loses a node or a leaf to a full list, or whose tree is deeper than the keys hold, is
+// marked and done by its own lane; the other jobs are whole.
+constexpr uint32_t kJobMask = 511u, kHeadMask = 8191u;
+constexpr int kJobBits = 9, kHeadBits = 13;  // job, then mesh (4 bits), then node or leaf
+template <int JOBS, int FRONT, int LEAVES>
+struct WalkLists {
+  uint32_t cnt[JOBS], seg[JOBS], fill[JOBS], lost[JOBS];
+  uint32_t front[2][FRONT];     // job | mesh | node
+  uint16_t fkey[2][FRONT];      // its path key
+  uint32_t leaf[LEAVES];        // as found: job | mesh | leaf
+  uint16_t key[LEAVES];         // its path key
+  uint16_t byjob[LEAVES];       // the entries above, by job
+  uint32_t njobs, nfront[sim::kWalkLevels + 1], nleaf;
 };
+constexpr int kWalkRayJobs = 144, kWalkRayFront = 384, kWalkRayLeaves = 400;
+constexpr int kWalkRayLane = 8;  // jobs of one lane (both cars)
+struct RayWalkSmem {
+  sim::RayMeshJob job[kWalkRayJobs];
+  Box3 jbox[kWalkRayJobs];
+  uint16_t jbody[kWalkRayJobs], jsd[kWalkRayJobs];
+  WalkLists<kWalkRayJobs, kWalkRayFront, kWalkRayLeaves> w;
+  sim::RayLeaf out[kWalkRayLeaves];
+  uint32_t at[kWalkRayLeaves];  // mesh | leaf << 4 of out[]
+};
+constexpr int kWalkPairJobs = 208, kWalkPairFront = 640, kWalkPairLeaves = 704;
+constexpr int kWalkPairLane = 8;   // jobs of one lane in one round
+constexpr int kWalkPairRounds = 3; // from this round on a job the lists lost is done by its lane alone
+constexpr int kWalkHits = 128;
+constexpr int kWalkSats = 48;      // SATs of a round whose feature pairs the block computes, kWalkFeat at a time
+constexpr int kWalkFeat = 15;
+struct PairJob {                   // a sim::LeafJob without what the static data holds
+  uint8_t kind, mesh, body;
+  union {
+    struct { Aff box_xf, mesh_to_box; };
+    struct { V3 center; float radius, rt, rt2; };
+  };
+};
+struct PairWalkSmem {
+  union {
+    PairJob job[kWalkPairJobs];
+    sim::FeatPair feat[kWalkFeat][sim::kPairs];  // over the job records, which nobody reads after the tests
+  };
+  Box3 jbox[kWalkPairJobs];
+  uint16_t jsd[kWalkPairJobs];
+  WalkLists<kWalkPairJobs, kWalkPairFront, kWalkPairLeaves> w;
+  sim::LeafHit hit[kWalkHits];
+  uint16_t at_tri[kWalkPairLeaves];  // in walk order: the leaf's triangle, and its hit's index + 1 (0: no contact)
+  uint16_t at_hit[kWalkPairLeaves];
+  sim::SatFront front[kWalkSats];
+  uint32_t front_at[kWalkSats];      // place | job << 16
+  uint32_t nsat, nhit;
+};
+static_assert(sizeof(sim::FeatPair) * kWalkFeat * sim::kPairs <= sizeof(PairJob) * kWalkPairJobs, "the feature pairs fit over the jobs");
+static_assert(sizeof(RayWalkSmem) + 256 <= 63 * 1024 && sizeof(PairWalkSmem) + 256 <= 63 * 1024, "a 64 KB carveout");
+static_assert(kWalkPairJobs <= 512 && kWalkRayJobs <= 512 && kMeshes <= 16 && kWalkPairLeaves < 65536 && kMaxTris < 65536 &&
+                  kWalkHits < 65535 && kMaxNodes < (1 << 19) && kMaxLeaves < (1 << 19),
+              "the lists' fields hold their values");
 // one shared buffer for the pools (they serve different pieces of the tick) and the prefix sums
 struct Pools {
   union {
     PoolSmem p3b;
     RayPoolSmem rays;
-    RayWalkSmem walk;
+    RayWalkSmem ray_walk;
+    PairWalkSmem pair_walk;
   };
   uint32_t warp_sum[32];
   uint32_t limit;
   uint32_t deferred;  // split 14: SATs of this round whose feature pairs the block computes
 };
-__device__ __forceinline__ Pools& pools() {
-  __shared__ Pools u;
-  return u;
-}
+extern __shared__ uint4 smem_pools[];  // sizeof(Pools) bytes for the splits that pool (9 on)
+__device__ __forceinline__ Pools& pools() { return *reinterpret_cast<Pools*>(smem_pools); }
 
 // block-wide exclusive prefix sum of v (every thread calls it); returns the exclusive sum, *total the block's sum
 __device__ __forceinline__ uint32_t block_scan(uint32_t v, uint32_t* total, Pools& sm) {
@@ -377,180 +422,395 @@ __device__ __noinline__ void rays_pooled(ArenaState& s, const StaticData* D, boo
   RSX_ZONE_END(zr5, 8);
 }
 
-// rays_pooled with the mesh walks pooled too (split 15); every thread of the block calls it.  Each lane's mesh
-// candidates (up to kRayJobsLane) become jobs in shared memory, the block walks all their BVHs level by level, sorts
-// each job's leaves into the stack walk's order, evaluates them, and each owner replays its candidates in order as in
-// rays_pooled.  Results equal vehicle_rays'.
-__device__ __noinline__ void rays_pooled_walk(ArenaState& s, const StaticData* D, bool act, int ci, sim::WheelHit hits[kWheels]) {
-  Pools& u = pools();
-  RayWalkSmem& sm = u.walk;
-  sim::RayPacket pk;
-  uint32_t cand[kHandles];
-  int nk = 0;
-  RSX_ZONE_BEGIN(zr0);
-  if (act) {
-    sim::vehicle_rays_begin(s, *D, ci, pk);
-    nk = sim::grid_candidates(s, *D, &pk, cand);
-  }
-  uint8_t jcand[kRayJobsLane];
-  int nj = 0;
-  for (int k = 0; k < nk; ++k) {
-    const uint32_t shape = D->bodies[cand[k]].shape;
-    if (shape == sim::SHAPE_BOX || shape == sim::SHAPE_SPHERE || shape == sim::SHAPE_PLANE) continue;
-    if (nj == kRayJobsLane) {  // more mesh bodies than a lane may pool: this lane walks its own
-      nj = -1;
-      break;
-    }
-    jcand[nj++] = (uint8_t)k;
-  }
-  const bool mine = nj > 0;
-  if (nj < 0) nj = 0;
-  RSX_ZONE_END(zr0, 5);
-  RSX_ZONE_BEGIN(zr1);
-  uint32_t total;
-  const uint32_t slot = block_scan((uint32_t)nj, &total, u);
-  // pooled lanes are a prefix in scan order, so the jobs are slots [0, limit)
-  const bool pooled = mine && slot + (uint32_t)nj <= (uint32_t)kRayJobs;
-  if (threadIdx.x == 0) {
-    for (int l = 0; l <= sim::kWalkLevels; ++l) sm.nfront[l] = 0;
-    sm.nleaf = 0;
-    sm.ovf = 0;
-  }
-  if (pooled) {
-    for (int j = 0; j < nj; ++j) {  // no body has been tested yet: the packet's fractions are all still 1
-      const uint32_t w = cand[jcand[j]], q = slot + (uint32_t)j;
-      sim::LocalRays lr;
-      sim::RayBox rb;
-      sim::ray_body_setup(s, *D, w, &pk, lr, rb);
-      sim::ray_mesh_job(lr, rb, sm.job[q]);
-      sm.jd[q] = D;
-      sm.jbox[q] = rb.box;
-      sm.jbody[q] = w;
-      sm.cnt[q] = 0;
-      sm.fill[q] = 0;
-    }
-    atomicMax(&u.limit, slot + (uint32_t)nj);
-  }
-  __syncthreads();
-  RSX_ZONE_END(zr1, 8);
-  RSX_ZONE_BEGIN(zr6);
-  const uint32_t J = u.limit;
-  // the jobs' meshes: every mesh of the job's body whose root box meets the job's box, in mesh order by key
-  for (uint32_t i = threadIdx.x; i < J * (uint32_t)kMeshes; i += blockDim.x) {
-    const uint32_t q = i / (uint32_t)kMeshes;
-    const int m = (int)(i % (uint32_t)kMeshes);
-    const StaticData& Dj = *sm.jd[q];
-    if (Dj.meshes[m].body == sm.jbody[q] && box_overlap(sm.jbox[q], Dj.meshes[m].root_box)) {
-      const uint32_t f = atomicAdd(&sm.nfront[0], 1u);
-      if (f < (uint32_t)kRayFront) {
-        sm.front[0][f][0] = q | ((uint32_t)m << 6);
-        sm.front[0][f][1] = sim::walk_root_key(m);
-      } else {
-        sm.ovf = 1;
-      }
-    }
-  }
-  __syncthreads();
+// The levels of a walk and the order of its leaves (split 15; every thread of the block calls it, after a barrier behind
+// the jobs' writes).  box(q): job q's box; expand(item, key, level, emit): the children of a front item whose boxes meet
+// the job's; keep(entry): whether a leaf entry is kept.  Afterwards each kept leaf's entry is in byjob[seg[q] ..
+// seg[q] + cnt[q]) of its job, in no order: rank_of gives its place in the stack walk's order.
+template <int JOBS, int FRONT, int LEAVES, class Expand, class Keep>
+__device__ __forceinline__ void walk_levels(WalkLists<JOBS, FRONT, LEAVES>& w, Expand&& expand, Keep&& keep) {
   for (int level = 0; level < sim::kWalkLevels; ++level) {
-    const uint32_t F = sm.nfront[level];
-    if (F == 0 || sm.ovf) break;  // (uniform: read after the barrier, written only between barriers)
+    const uint32_t F = min(w.nfront[level], (uint32_t)FRONT);
+    if (F == 0) break;  // (uniform: written only before the barrier above)
     const int cur = level & 1;
     for (uint32_t i = threadIdx.x; i < F; i += blockDim.x) {
-      const uint32_t it = sm.front[cur][i][0], key = sm.front[cur][i][1];
-      const uint32_t q = it & 63u, m = (it >> 6) & 15u, node = it >> 10;
-      sim::walk_expand(*sm.jd[q], (int)m, node, key, level, sm.jbox[q], [&](uint32_t ch, uint32_t k2) {
+      const uint32_t it = w.front[cur][i], head = it & kHeadMask, q = it & kJobMask;
+      expand(it, w.fkey[cur][i], level, [&](uint32_t ch, uint32_t key) {
         if (ch & 0x80000000u) {
-          const uint32_t e = atomicAdd(&sm.nleaf, 1u);
-          if (e < (uint32_t)kRayPairs) {
-            sm.leaf_a[e] = q | (m << 6) | ((ch & 0x7FFFFFFFu) << 10);
-            sm.key_a[e] = k2;
-            atomicAdd(&sm.cnt[q], 1u);
+          const uint32_t entry = head | ((ch & 0x7FFFFFFFu) << kHeadBits);
+          if (!keep(entry)) return;
+          const uint32_t e = atomicAdd(&w.nleaf, 1u);
+          if (e < (uint32_t)LEAVES) {
+            w.leaf[e] = entry;
+            w.key[e] = (uint16_t)key;
+            atomicAdd(&w.cnt[q], 1u);
           } else {
-            sm.ovf = 1;
+            w.lost[q] = 1;
           }
+        } else if (level + 1 == sim::kWalkLevels) {
+          w.lost[q] = 1;
         } else {
-          const uint32_t f = atomicAdd(&sm.nfront[level + 1], 1u);
-          if (f < (uint32_t)kRayFront) {
-            sm.front[cur ^ 1][f][0] = q | (m << 6) | (ch << 10);
-            sm.front[cur ^ 1][f][1] = k2;
+          const uint32_t f = atomicAdd(&w.nfront[level + 1], 1u);
+          if (f < (uint32_t)FRONT) {
+            w.front[cur ^ 1][f] = head | (ch << kHeadBits);
+            w.fkey[cur ^ 1][f] = (uint16_t)key;
           } else {
-            sm.ovf = 1;
+            w.lost[q] = 1;
           }
         }
       });
     }
     __syncthreads();
   }
-  // past a list's capacity, or a tree deeper than the keys hold: every lane walks its own this round
-  const bool walked = !(sm.ovf || sm.nfront[sim::kWalkLevels] != 0);
-  const uint32_t nl = walked ? sm.nleaf : 0u;
-  if (walked) {
-    if (threadIdx.x == 0) {
-      uint32_t acc = 0;
-      for (uint32_t q = 0; q < J; ++q) {
-        sm.seg[q] = acc;
-        acc += sm.cnt[q];
+  if (threadIdx.x < 32) {  // seg: the exclusive prefix sum of cnt
+    const uint32_t J = min(w.njobs, (uint32_t)JOBS);
+    uint32_t base = 0;
+    for (uint32_t q0 = 0; q0 < J; q0 += 32) {
+      const uint32_t q = q0 + threadIdx.x, c = q < J ? w.cnt[q] : 0u;
+      uint32_t x = c;
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, d);
+        if (threadIdx.x >= (uint32_t)d) x += y;
       }
+      if (q < J) w.seg[q] = base + x - c;
+      base += __shfl_sync(0xFFFFFFFFu, x, 31);
     }
-    __syncthreads();
-    for (uint32_t e = threadIdx.x; e < nl; e += blockDim.x) {
-      const uint32_t q = sm.leaf_a[e] & 63u;
-      const uint32_t at = sm.seg[q] + atomicAdd(&sm.fill[q], 1u);
-      sm.leaf_b[at] = sm.leaf_a[e];
-      sm.key_b[at] = sm.key_a[e];
-    }
-    __syncthreads();
-    for (uint32_t q = threadIdx.x; q < J; q += blockDim.x) {  // each job's leaves into key order
-      const uint32_t b = sm.seg[q], n = sm.cnt[q];
-      for (uint32_t i = 1; i < n; ++i) {
-        const uint32_t lv = sm.leaf_b[b + i], kv = sm.key_b[b + i];
-        uint32_t j = i;
-        for (; j > 0 && sm.key_b[b + j - 1] > kv; --j) {
-          sm.leaf_b[b + j] = sm.leaf_b[b + j - 1];
-          sm.key_b[b + j] = sm.key_b[b + j - 1];
-        }
-        sm.leaf_b[b + j] = lv;
-        sm.key_b[b + j] = kv;
-      }
-    }
-    __syncthreads();
   }
-  RSX_ZONE_END(zr6, 9);
-  RSX_ZONE_BEGIN(zr2);
-  for (uint32_t e = threadIdx.x; e < nl; e += blockDim.x) {
-    const uint32_t v = sm.leaf_b[e], q = v & 63u;
-    const StaticData& Dj = *sm.jd[q];
-    sim::ray_leaf_eval(sm.job[q], Dj, Dj.meshes[(v >> 6) & 15u], v >> 10, nullptr, &sm.out[e]);
-  }
-  RSX_ZONE_END(zr2, 6);
-  RSX_ZONE_BEGIN(zr3);
   __syncthreads();
-  RSX_ZONE_END(zr3, 8);
-  RSX_ZONE_BEGIN(zr4);
-  if (act) {
-    int j = 0;
-    for (int k = 0; k < nk; ++k) {
-      const uint32_t w = cand[k];
-      if (walked && pooled && j < nj && jcand[j] == k) {
-        sim::LocalRays lr;
-        sim::RayBox rb;
-        sim::ray_body_setup(s, *D, w, &pk, lr, rb);
-        const uint32_t q = slot + (uint32_t)j, b = sm.seg[q], n = sm.cnt[q];
-        for (uint32_t t = 0; t < n; ++t) {
-          const uint32_t v = sm.leaf_b[b + t];
-          sim::ray_leaf_replay(&lr, rb.lmax, *D, D->meshes[(v >> 6) & 15u], v >> 10, sm.out[b + t]);
+  const uint32_t nl = min(w.nleaf, (uint32_t)LEAVES);
+  for (uint32_t e = threadIdx.x; e < nl; e += blockDim.x) {
+    const uint32_t q = w.leaf[e] & kJobMask;
+    w.byjob[w.seg[q] + atomicAdd(&w.fill[q], 1u)] = (uint16_t)e;
+  }
+  __syncthreads();
+}
+// the place of leaf entry e of job q among the block's leaves: its job's segment, then the number of lower keys there
+// (a job's keys are distinct: a key is the path to the leaf)
+template <class Lists>
+__device__ __forceinline__ uint32_t rank_of(const Lists& w, uint32_t e, uint32_t q) {
+  const uint32_t b = w.seg[q], n = w.cnt[q], key = w.key[e];
+  uint32_t at = b;
+  for (uint32_t i = 0; i < n; ++i) at += w.key[w.byjob[b + i]] < key ? 1u : 0u;
+  return at;
+}
+template <class Lists>
+__device__ __forceinline__ void lists_clear(Lists& w) {
+  for (uint32_t q = threadIdx.x; q < sizeof(w.cnt) / 4; q += blockDim.x) w.cnt[q] = w.fill[q] = w.lost[q] = 0;
+  if (threadIdx.x <= (uint32_t)sim::kWalkLevels) w.nfront[threadIdx.x] = 0;
+  if (threadIdx.x == 0) w.njobs = w.nleaf = 0;
+}
+
+// The wheel rays of both cars of the thread's arena (act[ci]) in one round (split 15); every thread of the block calls
+// it.  The rays read poses, flags and static data only, and between car 0's rays and car 1's the tick changes none that
+// car 1's rays read: car 0's response writes velocities and wheel states, and car 1's pre-tick head moves a car only when
+// it respawns, which casts no rays; so both cars' rays can be cast after car 0's head.  Each lane lists the mesh bodies
+// among its candidates as jobs, the block walks them and evaluates their leaves, and each owner runs its candidates in
+// order, replaying the mesh ones.  Results equal vehicle_rays'.
+// What bounds it: the barriers behind the slowest lane's candidate search and replays, and the walk's levels.  One round
+// for both cars pays them once: with a round per car it took 414 thousand cycles a tick, together 316 thousand (65,536
+// arenas, 448 threads, of 2.97 and 2.48 million in all).
+__device__ __noinline__ void rays_walk_both(ArenaState& s, const StaticData* sds, uint32_t di, bool act0, bool act1, sim::WheelHit hits[kCars][kWheels]) {
+  Pools& u = pools();
+  RayWalkSmem& sm = u.ray_walk;
+  const StaticData* D = sds + di;
+  lists_clear(sm.w);
+  __syncthreads();
+  sim::RayPacket pk[kCars];
+  uint32_t cand[kCars][kHandles];
+  int nk[kCars] = {0, 0};
+  uint32_t jslot[kWalkRayLane];  // job | candidate << 16 | car << 24
+  int nj = 0;
+  RSX_ZONE_BEGIN(zr0);
+#pragma unroll 1
+  for (int ci = 0; ci < kCars; ++ci) {
+    if (!(ci ? act1 : act0)) continue;
+    sim::vehicle_rays_begin(s, *D, ci, pk[ci]);
+    nk[ci] = sim::grid_candidates(s, *D, &pk[ci], cand[ci]);
+    for (int k = 0; k < nk[ci] && nj < kWalkRayLane; ++k) {
+      const uint32_t w = cand[ci][k], shape = D->bodies[w].shape;
+      if (shape == sim::SHAPE_BOX || shape == sim::SHAPE_SPHERE || shape == sim::SHAPE_PLANE) continue;
+      const uint32_t q = atomicAdd(&sm.w.njobs, 1u);
+      if (q >= (uint32_t)kWalkRayJobs) break;  // past the pool: this lane walks the rest itself
+      jslot[nj++] = q | ((uint32_t)k << 16) | ((uint32_t)ci << 24);
+      sim::LocalRays lr;  // no body has been tested yet: the packet's fractions are all still 1
+      sim::RayBox rb;
+      sim::ray_body_setup(s, *D, w, &pk[ci], lr, rb);
+      sim::ray_mesh_job(lr, rb, sm.job[q]);
+      sm.jsd[q] = (uint16_t)di;
+      sm.jbox[q] = rb.box;
+      sm.jbody[q] = (uint16_t)w;
+    }
+  }
+  RSX_ZONE_END(zr0, 5);
+  RSX_ZONE_BEGIN(zr1);
+  __syncthreads();
+  RSX_ZONE_END(zr1, 8);
+  RSX_ZONE_BEGIN(zr6);
+  const uint32_t J = min(sm.w.njobs, (uint32_t)kWalkRayJobs);
+  if (J != 0) {  // (uniform: written only before the barrier)
+    // the jobs' meshes: every mesh of the job's body whose root box meets the job's box, in mesh order by key
+    for (uint32_t i = threadIdx.x; i < J * (uint32_t)kMeshes; i += blockDim.x) {
+      const uint32_t q = i / (uint32_t)kMeshes;
+      const int m = (int)(i % (uint32_t)kMeshes);
+      const StaticData& Dj = sds[sm.jsd[q]];
+      if (Dj.meshes[m].body == sm.jbody[q] && box_overlap(sm.jbox[q], Dj.meshes[m].root_box)) {
+        const uint32_t f = atomicAdd(&sm.w.nfront[0], 1u);
+        if (f < (uint32_t)kWalkRayFront) {
+          sm.w.front[0][f] = q | ((uint32_t)m << kJobBits);
+          sm.w.fkey[0][f] = (uint16_t)sim::walk_root_key(m);
+        } else {
+          sm.w.lost[q] = 1;
         }
-        ++j;
-      } else {
-        sim::ray_body(s, *D, w, &pk);
       }
     }
-    sim::wheel_packet_hits(s, *D, pk, hits);
+    __syncthreads();
+    walk_levels(
+        sm.w,
+        [&](uint32_t it, uint32_t key, int level, auto&& emit) {
+          const uint32_t q = it & kJobMask;
+          sim::walk_expand(sds[sm.jsd[q]], (int)((it >> kJobBits) & 15u), it >> kHeadBits, key, level, sm.jbox[q], emit);
+        },
+        [](uint32_t) { return true; });
+    RSX_ZONE_END(zr6, 9);
+    RSX_ZONE_BEGIN(zr2);
+    const uint32_t nl = min(sm.w.nleaf, (uint32_t)kWalkRayLeaves);
+    for (uint32_t e = threadIdx.x; e < nl; e += blockDim.x) {
+      const uint32_t v = sm.w.leaf[e], q = v & kJobMask, m = (v >> kJobBits) & 15u;
+      const uint32_t at = rank_of(sm.w, e, q);
+      const StaticData& Dj = sds[sm.jsd[q]];
+      sim::ray_leaf_eval(sm.job[q], Dj, Dj.meshes[m], v >> kHeadBits, nullptr, &sm.out[at]);
+      sm.at[at] = v >> kJobBits;
+    }
+    RSX_ZONE_END(zr2, 6);
+    RSX_ZONE_BEGIN(zr3);
+    __syncthreads();
+    RSX_ZONE_END(zr3, 8);
+  }
+  RSX_ZONE_BEGIN(zr4);
+  int j = 0;
+#pragma unroll 1
+  for (int ci = 0; ci < kCars; ++ci) {
+    if (!(ci ? act1 : act0)) continue;
+    for (int k = 0; k < nk[ci]; ++k) {
+      const uint32_t w = cand[ci][k];
+      const uint32_t slot = j < nj ? jslot[j] : ~0u, q = slot & kJobMask;
+      if ((slot >> 16) == ((uint32_t)k | ((uint32_t)ci << 8))) {
+        ++j;
+        if (!sm.w.lost[q]) {
+          sim::LocalRays lr;
+          sim::RayBox rb;
+          sim::ray_body_setup(s, *D, w, &pk[ci], lr, rb);
+          const uint32_t b = sm.w.seg[q], n = sm.w.cnt[q];
+          for (uint32_t t = 0; t < n; ++t) {
+            const uint32_t v = sm.at[b + t];
+            sim::ray_leaf_replay(&lr, rb.lmax, *D, D->meshes[v & 15u], v >> 4, sm.out[b + t]);
+          }
+          continue;
+        }
+      }
+      sim::ray_body(s, *D, w, &pk[ci]);
+    }
+    sim::wheel_packet_hits(s, *D, pk[ci], hits[ci]);
   }
   RSX_ZONE_END(zr4, 7);
   RSX_ZONE_BEGIN(zr5);
-  __syncthreads();  // the pool is read above: the next piece's writes come after every lane's reads
+  __syncthreads();  // the lists are read above: the next piece's writes come after every lane's reads
   RSX_ZONE_END(zr5, 8);
+}
+
+__device__ __forceinline__ sim::LeafJob leaf_job(const PairJob& p, const StaticData& D) {
+  sim::LeafJob j;
+  j.kind = p.kind;
+  j.tri_first = D.meshes[p.mesh].tri_first;
+  if (p.kind == sim::NEAR_BOX_JOB) {
+    const BodyConst& bc = D.bodies[p.body];
+    j.box_xf = p.box_xf;
+    j.mesh_to_box = p.mesh_to_box;
+    j.half = bc.box_half;
+    j.margin = bc.box_margin;
+    j.maxd = fadd(bc.box_margin, rmin(bc.breaking_threshold, D.bodies[p.mesh].breaking_threshold));
+  } else {
+    j.center = p.center;
+    j.radius = p.radius;
+    j.rt = p.rt;
+    j.rt2 = p.rt2;
+  }
+  return j;
+}
+
+// P3b of the thread's arena (have) with the tick's mesh jobs found, walked and tested before the pairs run (split 15);
+// every thread of the block calls it.  The jobs depend on nothing that P3b changes (sim/narrow.cuh near_peek), so each
+// lane lists its pairs' jobs, the block walks all of them level by level and tests their leaves (SAT feature pairs by the
+// whole block, kWalkFeat SATs at a time), and each owner then runs its pairs in order, adding the hits of each job it
+// opens.  A lane whose next job found no room waits for the next round.
+// What bounds it: the slowest lane's pairs, and the barriers around it.  p3b_pooled (split 14) needs a round per mesh pair
+// of the arena with the most (4.6 a tick on headline states), each as long as its slowest head and walk: 1,346 thousand
+// cycles a tick; here 892 thousand (65,536 arenas).  The lists are sized for a 64 KB carveout, which holds the 131 jobs
+// (at most 182 seen), 345 leaves and 39 hits a block has on headline states; twice the lists in 118 KB saved a round on
+// contact-heavy states but cost every phase L1 for the arenas' states: 12.55 against 11.7 - 11.9 ms a decision, and 24.0
+// against 20.5 - 21.5 ms on the contact-heavy mix.
+__device__ __noinline__ void p3b_walk_all(ArenaState& s, const StaticData* sds, uint32_t di, bool have, int* un) {
+  Pools& u = pools();
+  PairWalkSmem& sm = u.pair_walk;
+  const StaticData* D = sds + di;
+  sim::P3bLoop L;
+  bool more = have;
+  if (have) sim::p3b_begin(s, L);
+  for (int round = 0;; ++round) {
+    uint32_t listed = 0;            // the pairs listed
+    lists_clear(sm.w);
+    if (threadIdx.x == 0) sm.nsat = sm.nhit = 0;
+    RSX_ZONE_BEGIN(zb0);
+    __syncthreads();
+    RSX_ZONE_END(zb0, 56);
+    uint32_t jslot[kWalkPairLane];  // job | pair << 16
+    int nj = 0;
+    RSX_ZONE_BEGIN(zo);
+    if (more) {
+      for (uint32_t i = L.kind != sim::NEAR_DONE ? L.i - 1 : L.i; i < L.n && nj < kWalkPairLane; ++i) {
+        const Pair p = s.pairs[i];
+        sim::BoxJob bj;
+        sim::SphereJob sj;
+        const int kind = sim::near_peek(s, *D, D->proxies[p.h0].body, D->proxies[p.h1].body, bj, sj);
+        if (kind == sim::NEAR_DONE) continue;
+        const bool isbox = kind == sim::NEAR_BOX_JOB;
+        const uint32_t m = isbox ? bj.mesh_body : sj.mesh_body;
+        listed |= 1u << i;
+        if ((isbox ? bj.cu.n : sj.cu.n) == 0) continue;  // the mesh's root box is out of reach: no leaves
+        const uint32_t q = atomicAdd(&sm.w.njobs, 1u);
+        if (q >= (uint32_t)kWalkPairJobs) {
+          listed &= ~(1u << i);
+          break;
+        }
+        jslot[nj++] = q | (i << 16);
+        PairJob& job = sm.job[q];
+        job.kind = (uint8_t)kind;
+        job.mesh = (uint8_t)m;
+        if (isbox) {
+          job.body = (uint8_t)bj.car;
+          job.box_xf = bj.box_xf;
+          job.mesh_to_box = bj.mesh_to_box;
+        } else {
+          job.body = (uint8_t)sj.sph;
+          job.center = sj.center;
+          job.radius = sj.radius;
+          job.rt = sj.rt;
+          job.rt2 = sj.rt2;
+        }
+        sm.jsd[q] = (uint16_t)di;
+        sm.jbox[q] = isbox ? bj.box : sj.box;
+        const uint32_t f = atomicAdd(&sm.w.nfront[0], 1u);
+        sm.w.front[0][f] = q | (m << kJobBits);
+        sm.w.fkey[0][f] = 0;
+      }
+    }
+    RSX_ZONE_END(zo, 33);
+    LS_SYNC(56);
+    if (sm.w.njobs != 0) {  // (uniform: written only before the barrier)
+      RSX_ZONE_BEGIN(zw);
+      walk_levels(
+          sm.w,
+          [&](uint32_t it, uint32_t key, int level, auto&& emit) {
+            const uint32_t q = it & kJobMask;
+            sim::walk_expand(sds[sm.jsd[q]], (int)((it >> kJobBits) & 15u), it >> kHeadBits, key, level, sm.jbox[q], emit);
+          },
+          [&](uint32_t v) {
+            const uint32_t q = v & kJobMask;
+            if (sm.job[q].kind != sim::NEAR_BOX_JOB) return true;
+            const StaticData& Dj = sds[sm.jsd[q]];
+            const MeshInfo& m = Dj.meshes[(v >> kJobBits) & 15u];
+            return sim::tri_meets_box(Dj.tris[m.tri_first + Dj.leaves[m.leaf_first + (v >> kHeadBits)].tri], sm.jbox[q]);
+          });
+      RSX_ZONE_END(zw, 36);
+      auto put = [&](uint32_t at, uint32_t q, const sim::LeafHit& h) {
+        uint32_t i = 0;
+        if (h.found) {
+          i = atomicAdd(&sm.nhit, 1u) + 1;
+          if (i <= (uint32_t)kWalkHits) sm.hit[i - 1] = h;
+          else sm.w.lost[q] = 1;
+        }
+        sm.at_hit[at] = (uint16_t)(i <= (uint32_t)kWalkHits ? i : 0u);
+      };
+      RSX_ZONE_BEGIN(zt);
+      const uint32_t nl = min(sm.w.nleaf, (uint32_t)kWalkPairLeaves);
+      for (uint32_t e = threadIdx.x; e < nl; e += blockDim.x) {
+        const uint32_t v = sm.w.leaf[e], q = v & kJobMask;
+        const uint32_t at = rank_of(sm.w, e, q);
+        const StaticData& Dj = sds[sm.jsd[q]];
+        const uint32_t tri = Dj.leaves[Dj.meshes[(v >> kJobBits) & 15u].leaf_first + (v >> kHeadBits)].tri;
+        sm.at_tri[at] = (uint16_t)tri;
+        sim::LeafHit h;
+        sim::SatFront f;
+        if (!sim::leaf_test_front(leaf_job(sm.job[q], Dj), Dj, tri, &h, &f)) {
+          const uint32_t d = atomicAdd(&sm.nsat, 1u);
+          if (d < (uint32_t)kWalkSats) {  // the block computes its feature pairs below
+            sm.front[d] = f;
+            sm.front_at[d] = at | (q << 16);
+            continue;
+          }
+          sim::FeatPair P[sim::kPairs];  // past the list: this thread computes them itself
+          sim::enum_pairs(f.hu, f.q, f.e, P);
+          sim::leaf_test_back(f, P, &h);
+        }
+        put(at, q, h);
+      }
+      RSX_ZONE_END(zt, 34);
+      LS_SYNC(56);
+      const uint32_t ns = min(sm.nsat, (uint32_t)kWalkSats);
+      for (uint32_t d0 = 0; d0 < ns; d0 += (uint32_t)kWalkFeat) {  // (the pairs overlay the job records, which are read by now)
+        const uint32_t nd = min(ns - d0, (uint32_t)kWalkFeat);
+        RSX_ZONE_BEGIN(zf);
+        for (uint32_t w = threadIdx.x; w < nd * (uint32_t)sim::kPairs; w += blockDim.x) {
+          const uint32_t d = w / (uint32_t)sim::kPairs, i = w % (uint32_t)sim::kPairs;
+          sm.feat[d][i] = sim::feat_pair(sm.front[d0 + d], (int)i);
+        }
+        RSX_ZONE_END(zf, 34);
+        LS_SYNC(56);
+        RSX_ZONE_BEGIN(zg);
+        for (uint32_t d = threadIdx.x; d < nd; d += blockDim.x) {
+          sim::LeafHit h;
+          sim::leaf_test_back(sm.front[d0 + d], sm.feat[d], &h);
+          put(sm.front_at[d0 + d] & 0xFFFFu, sm.front_at[d0 + d] >> 16, h);
+        }
+        RSX_ZONE_END(zg, 34);
+        LS_SYNC(56);
+      }
+    }
+    RSX_ZONE_BEGIN(zc);
+    if (more) {
+      more = false;
+      for (int j = 0; j < nj; ++j)
+        if (sm.w.lost[jslot[j] & kJobMask]) listed &= ~(1u << (jslot[j] >> 16));
+      int j = 0;
+      while (sim::p3b_open(s, *D, L, listed) != sim::NEAR_DONE) {
+        const uint32_t pair = L.i - 1;
+        while (j < nj && (jslot[j] >> 16) < pair) ++j;
+        const bool has = j < nj && (jslot[j] >> 16) == pair;
+        if ((listed >> pair) & 1u) {
+          if (has) {
+            const uint32_t q = jslot[j] & kJobMask, b = sm.w.seg[q], n = sm.w.cnt[q];
+            for (uint32_t t = 0; t < n; ++t) {
+              const uint32_t i = sm.at_hit[b + t];
+              if (i != 0) sim::p3b_add_hit(s, *D, L, sm.at_tri[b + t], sm.hit[i - 1]);
+            }
+          }
+          L.walk_done = true;
+          sim::p3b_close(s, *D, L);
+        } else if (has && round >= kWalkPairRounds) {
+          sim::p3b_job_alone(s, *D, L);
+        } else {  // its job found no room: the next round
+          more = true;
+          break;
+        }
+      }
+    }
+    RSX_ZONE_END(zc, 35);
+    RSX_ZONE_BEGIN(zd);
+    const bool again = __syncthreads_or(more);  // (the lists are read above)
+    RSX_ZONE_END(zd, 56);
+    if (!again) break;
+  }
+  if (have && L.unimplemented != 0) *un = 1;
 }
 
 }  // namespace
@@ -558,49 +818,61 @@ __device__ __noinline__ void rays_pooled_walk(ArenaState& s, const StaticData* D
 template <int SPLIT>
 __global__ void __launch_bounds__(RSX_LS_MAXT, 1) K_NAME(uint32_t* states, const StaticData* sds, const uint8_t* sd_index,
                                                         const Controls* controls, uint32_t* result, uint32_t* ev_or,
-                                                        const uint32_t* order, uint32_t* counter, uint32_t n, uint32_t t_first,
-                                                        uint32_t t_last) {
+                                                        const uint32_t* order, uint32_t* counter, uint32_t n, uint32_t width,
+                                                        uint32_t t_first, uint32_t t_last) {
   const uint32_t lane = threadIdx.x & 31u;
   ArenaState s;
   Controls c0, c1;
   const StaticData* D = sds;
-  uint32_t a = 0, t = 0, scored = 0, unimpl = 0, ev = 0;
-  bool live = false, have = false, ovf = false;
+  uint32_t a = 0, di = 0, t = 0, scored = 0, unimpl = 0, ev = 0;
+  // without a queue the claims are dealt out evenly: over the identity order each block's in a row (neighbouring arenas on
+  // one SM: 2% faster at 65,536 arenas than the blocks in turn), over another order the blocks in turn (its costliest
+  // arenas come first)
+  const uint32_t nw = blockDim.x >> 5, warp = threadIdx.x >> 5, claims = (n + width - 1) / width;
+  const uint32_t first = order ? blockIdx.x : (uint32_t)((uint64_t)claims * blockIdx.x / gridDim.x), step = order ? gridDim.x : 1u;
+  const uint32_t end = order ? claims : (uint32_t)((uint64_t)claims * (blockIdx.x + 1) / gridDim.x);
+  uint32_t next = first + warp * step;
+  bool busy = false;               // the warp holds a claim (uniform over the warp)
+  bool have = false, ovf = false;  // the lane steps an arena
   for (;;) {
-    // a warp without arenas claims the next 32 entries of the queue
-    if (!have) {
+    // a warp without arenas claims its next ones
+    if (!busy) {
       uint32_t base = 0;
-      if (lane == 0) base = atomicAdd(counter, 32u);
-      base = __shfl_sync(0xFFFFFFFFu, base, 0);
+      if (counter) {
+        if (lane == 0) base = atomicAdd(counter, width);
+        base = __shfl_sync(0xFFFFFFFFu, base, 0);
+      } else {
+        base = next < end ? next * width : n;
+        next += nw * step;
+      }
       if (base < n) {
-        uint32_t i = base + lane;
-        live = i < n;
-        uint32_t j = live ? i : base;
-        a = order ? order[j] : j;
-        if (a >= n) {  // an order entry past n (not a permutation): step arena 0 as a copy and store nothing
-          a = 0;
-          live = false;
-        }
-        D = sds + (sd_index ? sd_index[a] : 0);
-        RSX_ZONE_BEGIN(zl);
-        load_tick(&s, states, a);
-        RSX_ZONE_END(zl, 60);
-        c0 = controls[(size_t)a * kCars];
-        c1 = controls[(size_t)a * kCars + 1];
+        busy = true;
         t = t_first;
-        scored = unimpl = ev = 0;
-        if (t_first > 1) {  // a later launch of a split decision: the progress so far rides in the result / event words
-          uint32_t r0 = result[a];
-          scored = r0 & kScoredMask;
-          unimpl = r0 & kUnimplemented;
-          ev = ev_or ? ev_or[a] : 0u;
-          if (scored) live = false;  // decided in an earlier launch (the buffer holds its goal state): store nothing
+        const uint32_t i = base + lane;
+        a = lane < width && i < n ? (order ? order[i] : i) : n;
+        // (a lane past the claim's arenas, or at an order entry past n (not a permutation), steps nothing)
+        if (a < n) {
+          have = true;
+          di = sd_index ? sd_index[a] : 0;
+          D = sds + di;
+          RSX_ZONE_BEGIN(zl);
+          load_tick(&s, states, a);
+          RSX_ZONE_END(zl, 60);
+          c0 = controls[(size_t)a * kCars];
+          c1 = controls[(size_t)a * kCars + 1];
+          scored = unimpl = ev = 0;
+          if (t_first > 1) {  // a later launch of a split decision: the progress so far rides in the result / event words
+            uint32_t r0 = result[a];
+            scored = r0 & kScoredMask;
+            unimpl = r0 & kUnimplemented;
+            ev = ev_or ? ev_or[a] : 0u;
+            if (scored) have = false;  // decided in an earlier launch: the buffer holds its goal state
+          }
+          ovf = false;
         }
-        ovf = false;
-        have = true;
       }
     }
-    if (!__syncthreads_or(have)) break;
+    if (!__syncthreads_or(busy)) break;
     // one tick, phase by phase in lockstep (every thread reaches every barrier)
     int un = 0;
     if (have) {
@@ -618,6 +890,50 @@ __global__ void __launch_bounds__(RSX_LS_MAXT, 1) K_NAME(uint32_t* states, const
         sim::flip_zdamp(s, *D, 0);
         sim::flip_zdamp(s, *D, 1);
       }
+      if (SPLIT >= 15) {
+        // P1: car 0's head, both cars' wheel rays, car 0's response, car 1's head and response
+        bool act0 = false, act1 = false;
+        float thr0 = 0.0f, thr1 = 0.0f;
+        uint32_t was0 = 0, was1 = 0;
+        {
+          RSX_ZONE_BEGIN(z1);
+          if (have) {
+            was0 = s.cars[0].on_ground;
+            act1 = !s.cars[1].is_demoed;
+            act0 = sim::car_pre_tick_head(s, *D, 0, &thr0);
+          }
+          RSX_ZONE_END(z1, 41);
+        }
+        LS_SYNC(51);
+        sim::WheelHit hits[kCars][kWheels];
+        {
+          RSX_ZONE_BEGIN(z2);
+          rays_walk_both(s, sds, di, act0, act1, hits);
+          RSX_ZONE_END(z2, 42);
+        }
+#pragma unroll 1
+        for (int ci = 0; ci < kCars; ++ci) {
+          if (ci) {
+            RSX_ZONE_BEGIN(z1);
+            if (have) {
+              was1 = s.cars[1].on_ground;
+              act1 = sim::car_pre_tick_head(s, *D, 1, &thr1);
+            }
+            RSX_ZONE_END(z1, 41);
+            LS_SYNC(51);
+          }
+          RSX_ZONE_BEGIN(z3);
+          if (have) {
+            if (ci ? act1 : act0) {
+              sim::vehicle_response(s, *D, ci, sim::kTickTime, s.cars[ci].handbrake_val, ci ? thr1 : thr0, D->cars[ci].three_wheels != 0, hits[ci]);
+              sim::car_pre_tick_tail(s, *D, ci);
+            }
+            if (!(ci ? was1 : was0) && s.cars[ci].on_ground) s.events |= 1u << (EV_LANDED + ci);
+          }
+          RSX_ZONE_END(z3, 43);
+          LS_SYNC(53);
+        }
+      } else
 #pragma unroll 1
       for (int ci = 0; ci < kCars; ++ci) {
         // P1 for car ci in three barrier-separated parts: pre-tick head, wheel rays, wheel response + tail
@@ -644,9 +960,7 @@ __global__ void __launch_bounds__(RSX_LS_MAXT, 1) K_NAME(uint32_t* states, const
         sim::WheelHit hits[kWheels];
         {
           RSX_ZONE_BEGIN(z2);
-          if (SPLIT >= 15)
-            rays_pooled_walk(s, D, have && act, ci, hits);
-          else if (SPLIT >= 10)
+          if (SPLIT >= 10)
             rays_pooled(s, D, have && act, ci, hits);
           else if (have && act)
             sim::vehicle_rays(s, *D, ci, hits);
@@ -720,7 +1034,10 @@ __global__ void __launch_bounds__(RSX_LS_MAXT, 1) K_NAME(uint32_t* states, const
           continue;
         }
         if (SPLIT >= 9 && k == 4) {  // P3b with the block's leaf tests pooled
-          p3b_pooled<(SPLIT >= 14)>(s, D, have, &un);
+          if (SPLIT >= 15)
+            p3b_walk_all(s, sds, di, have, &un);
+          else
+            p3b_pooled<(SPLIT >= 14)>(s, D, have, &un);
           continue;
         }
         if (SPLIT == 3 && k == 4) {
@@ -775,36 +1092,42 @@ __global__ void __launch_bounds__(RSX_LS_MAXT, 1) K_NAME(uint32_t* states, const
         ev |= s.events;
         if (sim::ball_scored(s, *D)) {
           scored = t;
-          if (live) store_tick(states, a, &s);
+          store_tick(states, a, &s);
           ovf = sim::any_overflow(s);
         }
       }
       if (t == t_last) {  // the end of this launch's ticks (tick 8: of the decision)
         RSX_ZONE_BEGIN(zs);
         if (scored == 0) {
-          if (live) store_tick(states, a, &s);
+          store_tick(states, a, &s);
           ovf = sim::any_overflow(s);
         }
         RSX_ZONE_END(zs, 61);
-        if (live) {
-          if (ev_or) ev_or[a] = ev;
-          result[a] = scored | unimpl | (ovf ? kOverflow : 0u);
-        }
-        have = false;
+        if (ev_or) ev_or[a] = ev;
+        result[a] = scored | unimpl | (ovf ? kOverflow : 0u);
       }
-      ++t;
     }
+    if (busy && t++ == t_last) busy = have = false;
   }
 }
 
 cudaError_t L_NAME(uint32_t* states, const void* sds, const uint8_t* sd_index, const void* controls, uint32_t* result, uint32_t* ev_or,
-                   const uint32_t* order, uint32_t* counter, uint32_t n, uint32_t grid, uint32_t block, int split, uint32_t t_first,
-                   uint32_t t_last, cudaStream_t s) {
+                   const uint32_t* order, uint32_t* counter, uint32_t n, uint32_t width, uint32_t grid, uint32_t block, int split,
+                   uint32_t t_first, uint32_t t_last, cudaStream_t s) {
   const StaticData* D = (const StaticData*)sds;
   const Controls* C = (const Controls*)controls;
-#define RSX_LS_LAUNCH(k) K_NAME<k><<<grid, block, 0, s>>>(states, D, sd_index, C, result, ev_or, order, counter, n, t_first, t_last)
+  const size_t pool = split >= 9 ? sizeof(Pools) : 0;
+#define RSX_LS_LAUNCH(k)                                                                                              \
+  if (pool) {                                                                                                         \
+    const cudaError_t e = cudaFuncSetAttribute(K_NAME<k>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pool);    \
+    if (e != cudaSuccess) return e;                                                                                   \
+  }                                                                                                                   \
+  K_NAME<k><<<grid, block, pool, s>>>(states, D, sd_index, C, result, ev_or, order, counter, n, width, t_first, t_last)
   switch (split) {
     case 15: RSX_LS_LAUNCH(15); break;
+#ifdef RSX_LS_WIDE_REGS
+    default: return cudaErrorInvalidValue;
+#else
     case 14: RSX_LS_LAUNCH(14); break;
     case 11: RSX_LS_LAUNCH(11); break;
     case 10: RSX_LS_LAUNCH(10); break;
@@ -818,6 +1141,7 @@ cudaError_t L_NAME(uint32_t* states, const void* sds, const uint8_t* sd_index, c
     case 2: RSX_LS_LAUNCH(2); break;
     case 1: RSX_LS_LAUNCH(1); break;
     default: RSX_LS_LAUNCH(0); break;
+#endif
   }
 #undef RSX_LS_LAUNCH
   return cudaGetLastError();
@@ -834,7 +1158,7 @@ extern "C" int rsx_zones_lockstep(uint32_t* d_states, uint32_t n, const void* d_
   if (cudaMemset(d_counter, 0, 4) != cudaSuccess) return -2;
   int sms = 0;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, 0);
-  if (L_NAME(d_states, d_statics, d_sd_index, d_controls, d_result, nullptr, nullptr, d_counter, n, sms < 148 ? sms : 148, block, split, 1,
+  if (L_NAME(d_states, d_statics, d_sd_index, d_controls, d_result, nullptr, nullptr, d_counter, n, 32, sms < 148 ? sms : 148, block, split, 1,
              kTicksPerDecision, 0) != cudaSuccess)
     return -2;
   if (cudaDeviceSynchronize() != cudaSuccess) return -2;

@@ -29,17 +29,27 @@ RSX_F void add_pair(ArenaState& S, const StaticData& D, uint32_t h0, uint32_t h1
   S.pairs[S.n_pairs++] = Pair{i0, i1};
 }
 
+// the pool index of the pair's manifold (either body order), or -1; four entries' bodies are read at a time, so that the
+// loads of a pool of manifolds (332 bytes apart in the state) overlap
+RSX_F int32_t find_manifold(const ArenaState& S, uint32_t b0, uint32_t b1) {
+  const uint32_t lo = b0 < b1 ? b0 : b1, hi = b0 < b1 ? b1 : b0;
+  for (uint32_t i = 0; i < S.n_manifolds && i < (uint32_t)kMaxManifolds; i += 4) {
+    static_assert(kMaxManifolds % 4 == 0, "whole groups");
+    uint32_t a[4], b[4];
+#pragma unroll
+    for (uint32_t j = 0; j < 4; ++j) {
+      a[j] = S.manifolds[i + j].body0;
+      b[j] = S.manifolds[i + j].body1;
+    }
+#pragma unroll
+    for (uint32_t j = 0; j < 4; ++j)
+      if (i + j < S.n_manifolds && (a[j] < b[j] ? a[j] : b[j]) == lo && (a[j] < b[j] ? b[j] : a[j]) == hi) return (int32_t)(i + j);
+  }
+  return -1;
+}
 // release_manifold of the pair (body0, body1): the active list loses the index, the pool's last manifold fills the hole
 RSX_F void release_manifold(ArenaState& S, uint32_t b0, uint32_t b1) {
-  uint32_t lo = b0 < b1 ? b0 : b1, hi = b0 < b1 ? b1 : b0;
-  int found = -1;
-  for (uint32_t i = 0; i < S.n_manifolds; ++i) {
-    uint32_t a = S.manifolds[i].body0, b = S.manifolds[i].body1;
-    if ((a < b ? a : b) == lo && (a < b ? b : a) == hi) {
-      found = (int)i;
-      break;
-    }
-  }
+  const int32_t found = find_manifold(S, b0, b1);
   if (found < 0) return;
   uint32_t idx = (uint32_t)found, last = S.n_manifolds - 1;
   uint32_t w = 0;

@@ -787,7 +787,8 @@ struct BoxJob {
   Cursor cu;
 };
 
-RSX_F bool sphere_job_begin(Ctx& c, uint32_t sph, uint32_t mb, int32_t mi, SphereJob& j) {
+// (cbt: the pair's breaking threshold; mi: its manifold's pool index)
+RSX_F bool sphere_job_begin(Ctx& c, uint32_t sph, uint32_t mb, int32_t mi, float cbt, SphereJob& j) {
   if (!(mb < (uint32_t)kMeshes && c.D.meshes[mb].body == mb)) {
     c.unimplemented += 1;
     return false;
@@ -795,7 +796,6 @@ RSX_F bool sphere_job_begin(Ctx& c, uint32_t sph, uint32_t mb, int32_t mi, Spher
   const MeshInfo* mesh = &c.D.meshes[mb];
   Aff xs = body_xf(c.S, c.D, sph), xm = body_xf(c.S, c.D, mb);
   V3 cis = xs.t - xm.t;
-  float cbt = breaking(c.D, c.S.manifolds[mi]);
   float r = c.D.bodies[sph].sphere_margin;
   float rt = fadd(r, cbt);
   j.manifold = mi;
@@ -839,12 +839,15 @@ RSX_F bool box_job_begin(Ctx& c, uint32_t car, uint32_t mb, BoxJob& j) {
   cursor_init(j.cu, *mesh, bt);
   return true;
 }
+// a box job's filter of the triangles its walk reaches
+RSX_F bool tri_meets_box(const Tri& t, const Box3& b) {
+  V3 lo = vmin(vmin(t.p0, t.p1), t.p2), hi = vmax(vmax(t.p0, t.p1), t.p2);
+  return all_le(lo, b.hi) && all_ge(hi, b.lo);
+}
 RSX_F bool box_job_next(const StaticData& D, BoxJob& j, uint32_t* tri) {
   uint32_t leaf;
   while (cursor_next(j.cu, D, *j.mesh, j.box, &leaf)) {
-    const Tri& t = D.tris[j.mesh->tri_first + leaf];
-    V3 lo = vmin(vmin(t.p0, t.p1), t.p2), hi = vmax(vmax(t.p0, t.p1), t.p2);
-    if (!(all_le(lo, j.box.hi) && all_ge(hi, j.box.lo))) continue;
+    if (!tri_meets_box(D.tris[j.mesh->tri_first + leaf], j.box)) continue;
     *tri = leaf;
     return true;
   }
@@ -852,14 +855,6 @@ RSX_F bool box_job_next(const StaticData& D, BoxJob& j, uint32_t* tri) {
 }
 
 // ---- the near callback ----
-RSX_F int32_t find_manifold(const ArenaState& S, uint32_t b0, uint32_t b1) {
-  uint32_t lo = b0 < b1 ? b0 : b1, hi = b0 < b1 ? b1 : b0;
-  for (uint32_t i = 0; i < S.n_manifolds; ++i) {
-    uint32_t a = S.manifolds[i].body0, b = S.manifolds[i].body1;
-    if ((a < b ? a : b) == lo && (a < b ? b : a) == hi) return (int32_t)i;
-  }
-  return -1;
-}
 RSX_F int32_t insert_manifold(ArenaState& S, const Manifold& m) {
   if (S.n_manifolds >= (uint32_t)kMaxManifolds) {
     S.overflow[OVF_MANIFOLDS] += 1;
@@ -907,8 +902,32 @@ RSX_HD RSX_NOINL inline void near_tail(Ctx& c, uint32_t rb0, uint32_t rb1, int32
 enum { NEAR_DONE = 0, NEAR_BOX_JOB = 1, NEAR_SPHERE_JOB = 2 };
 struct NearPair { uint32_t rb0, rb1; int32_t cached; };
 
-RSX_F int near_head(Ctx& c, uint32_t rb0, uint32_t rb1, NearPair& np, BoxJob& bj, SphereJob& sj) {
+// (found: near_peek found the pair's mesh job and the caller has its leaves tested already, so the head's own tests up to
+// the job hold and only what adding the hits needs is set up)
+RSX_F int near_head(Ctx& c, uint32_t rb0, uint32_t rb1, NearPair& np, BoxJob& bj, SphereJob& sj, bool found = false) {
   ArenaState& S = c.S;
+  if (found) {
+    const uint32_t cv = c.D.bodies[rb0].shape == SHAPE_MESH ? rb1 : rb0, mb = cv == rb0 ? rb1 : rb0;
+    np.rb0 = rb0;
+    np.rb1 = rb1;
+    np.cached = find_manifold(S, rb0, rb1);
+    if (c.D.bodies[cv].shape == SHAPE_BOX) {
+      bj.has_m = false;
+      bj.car = cv;
+      bj.mesh_body = mb;
+      bj.mesh = &c.D.meshes[mb];
+      bj.tri_rot = body_xf(S, c.D, mb).m;
+      return NEAR_BOX_JOB;
+    }
+    const int32_t pi = np.cached < 0 ? insert_manifold(S, manifold_new(cv, mb)) : np.cached;
+    if (pi < 0) return NEAR_DONE;
+    sj.manifold = pi;
+    sj.sph = cv;
+    sj.mesh_body = mb;
+    sj.mesh = &c.D.meshes[mb];
+    sj.mesh_t = body_xf(S, c.D, mb).t;
+    return NEAR_SPHERE_JOB;
+  }
   if ((!body_awake(S, c.D, rb0) && !body_awake(S, c.D, rb1)) || !body_responds(S, c.D, rb0) || !body_responds(S, c.D, rb1)) return NEAR_DONE;
   int32_t cached = find_manifold(S, rb0, rb1);
   np.rb0 = rb0;
@@ -936,7 +955,7 @@ RSX_F int near_head(Ctx& c, uint32_t rb0, uint32_t rb1, NearPair& np, BoxJob& bj
     if (pi < 0) pi = insert_manifold(S, manifold_new(cv, cc));
     if (pi < 0) return NEAR_DONE;
     RSX_ZONE_BEGIN(z_sj);
-    bool job = sphere_job_begin(c, cv, cc, pi, sj);
+    bool job = sphere_job_begin(c, cv, cc, pi, breaking(c.D, S.manifolds[pi]), sj);
     RSX_ZONE_END(z_sj, 21);
     if (job) return NEAR_SPHERE_JOB;
     push_active(S, (uint32_t)pi);
@@ -981,6 +1000,24 @@ RSX_F int near_head(Ctx& c, uint32_t rb0, uint32_t rb1, NearPair& np, BoxJob& bj
   return NEAR_DONE;
 }
 
+// The mesh job that the head of the pair (rb0, rb1) opens, without the head's side effects: fills bj or sj and returns
+// the job's kind, or NEAR_DONE when the head opens none.  A head reads, up to its job, the bodies' poses, flags and
+// activation and the static data, none of which P3b changes, so a job found here before any pair ran is the job the
+// head opens in its turn (unless the manifold pool is full by then: that head opens none).
+RSX_F int near_peek(ArenaState& S, const StaticData& D, uint32_t rb0, uint32_t rb1, BoxJob& bj, SphereJob& sj) {
+  const uint32_t k0 = D.bodies[rb0].shape, k1 = D.bodies[rb1].shape;
+  if (k0 != SHAPE_MESH && k1 != SHAPE_MESH) return NEAR_DONE;
+  const uint32_t cv = k0 == SHAPE_MESH ? rb1 : rb0, mb = k0 == SHAPE_MESH ? rb0 : rb1;
+  const uint32_t kc = D.bodies[cv].shape;
+  if (kc != SHAPE_SPHERE && kc != SHAPE_BOX) return NEAR_DONE;
+  if ((!body_awake(S, D, rb0) && !body_awake(S, D, rb1)) || !body_responds(S, D, rb0) || !body_responds(S, D, rb1)) return NEAR_DONE;
+  Ctx c = {S, D, 0};
+  if (kc == SHAPE_SPHERE)
+    return sphere_job_begin(c, cv, mb, -1, rmin(D.bodies[cv].breaking_threshold, D.bodies[mb].breaking_threshold), sj) ? NEAR_SPHERE_JOB : NEAR_DONE;
+  if (!box_overlap(child_box(S, D, cv), body_box(S, D, mb))) return NEAR_DONE;
+  return box_job_begin(c, cv, mb, bj) ? NEAR_BOX_JOB : NEAR_DONE;
+}
+
 // P3b driver: pairs in order; a mesh pair's leaves in BVH walk order, each leaf's contact added in that order.  The loop
 // is kept as a state (P3bLoop) and a step, so that a kernel can step the loops of many arenas in lockstep; phase3b runs
 // the steps to the end.  A step runs the pair heads up to the next mesh job (or the end of the pairs), then one chunk of
@@ -1010,14 +1047,15 @@ RSX_F void p3b_begin(const ArenaState& S, P3bLoop& L) {
 RSX_F bool p3b_more(const P3bLoop& L) { return L.kind != NEAR_DONE || L.i < L.n; }
 
 // The pair heads up to the next mesh job: returns its kind (NEAR_BOX_JOB / NEAR_SPHERE_JOB), or NEAR_DONE when the pairs
-// ran out.  A job already open is returned as it is.
-RSX_F int p3b_open(ArenaState& S, const StaticData& D, P3bLoop& L) {
+// ran out.  A job already open is returned as it is.  (found: bit i set when pair i's job is found and tested, near_head)
+RSX_F int p3b_open(ArenaState& S, const StaticData& D, P3bLoop& L, uint32_t found = 0) {
   if (L.kind != NEAR_DONE) return L.kind;
   Ctx c = {S, D, L.unimplemented};
   RSX_ZONE_BEGIN(z_head);
   while (L.i < L.n) {
+    const bool f = ((found >> L.i) & 1u) != 0;
     Pair p = S.pairs[L.i++];
-    L.kind = near_head(c, D.proxies[p.h0].body, D.proxies[p.h1].body, L.np, L.bj, L.sj);
+    L.kind = near_head(c, D.proxies[p.h0].body, D.proxies[p.h1].body, L.np, L.bj, L.sj, f);
     if (L.kind != NEAR_DONE) break;
   }
   RSX_ZONE_END(z_head, 10);
@@ -1179,10 +1217,8 @@ RSX_F void p3b_close(ArenaState& S, const StaticData& D, P3bLoop& L) {
   L.unimplemented = c.unimplemented;
 }
 
-// one step; false when the phase has no work left
-RSX_F bool p3b_step(ArenaState& S, const StaticData& D, P3bLoop& L) {
-  if (!p3b_more(L)) return false;
-  if (p3b_open(S, D, L) == NEAR_DONE) return false;
+// one chunk of the open job on the calling lane
+RSX_F void p3b_chunk(ArenaState& S, const StaticData& D, P3bLoop& L) {
   uint32_t tris[kLeafChunk];
   int k = p3b_collect(D, L, tris, kLeafChunk);
   LeafJob j;
@@ -1192,6 +1228,17 @@ RSX_F bool p3b_step(ArenaState& S, const StaticData& D, P3bLoop& L) {
     if (leaf_test(j, D, tris[i], &h)) p3b_add_hit(S, D, L, tris[i], h);
   }
   if (L.walk_done) p3b_close(S, D, L);
+}
+// the whole open job on the calling lane
+RSX_HD RSX_NOINL inline void p3b_job_alone(ArenaState& S, const StaticData& D, P3bLoop& L) {
+  while (L.kind != NEAR_DONE) p3b_chunk(S, D, L);
+}
+
+// one step; false when the phase has no work left
+RSX_F bool p3b_step(ArenaState& S, const StaticData& D, P3bLoop& L) {
+  if (!p3b_more(L)) return false;
+  if (p3b_open(S, D, L) == NEAR_DONE) return false;
+  p3b_chunk(S, D, L);
   return p3b_more(L);
 }
 
