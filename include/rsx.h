@@ -75,7 +75,8 @@ int rsx_copy_raw(void* d_dst, const void* d_src, uint64_t bytes, void* stream);
 
 /* ---- the decision (SimDevice::sim8, device.rs:155-168; kernel sim.cu:95-104) ----
  * One decision of every arena in place: 8 ticks with controls[a*2+i] (device memory, 16 words per arena), result[a] the
- * scored tick | RSX_UNIMPLEMENTED | RSX_OVERFLOW (device memory).  block: 1..64 threads (RSX_SIM8_BLOCK in production).
+ * scored tick | RSX_UNIMPLEMENTED | RSX_OVERFLOW (device memory).  block: 1..64 threads (RSX_SIM8_BLOCK in production); a
+ * call of at most one arena per SM without a trace is launched in a shape of the library's own (same words).
  * trace: null, or 8 AoSoA buffers (8 * rsx_aosoa_words(n) words, device memory) that receive the state after each tick. */
 int rsx_sim8(rsx_device* dev, rsx_states* st, rsx_static* sd, const rsx_controls* d_controls, uint32_t* d_result, uint32_t block,
              uint32_t* d_trace);
@@ -89,7 +90,8 @@ int rsx_phase(rsx_device* dev, int k, rsx_states* st, rsx_static* sd, int32_t* d
 int rsx_identity(rsx_device* dev, const uint32_t* d_in, uint32_t* d_out, uint32_t n, int tick_only);
 
 /* ---- extensions (no counterpart in the reference's kernel set; the functions above are unchanged by them) ----
- * Per-arena car pairing: d_static points at `count` StaticData, sd_index[a] (u8, device memory) selects arena a's. */
+ * Per-arena car pairing: d_static points at `count` StaticData, sd_index[a] (u8, device memory) selects arena a's.  Up to
+ * 256 arenas per SM the call runs the lockstep kernel below in a shape of the library's own (same words). */
 int rsx_sim8_multi_raw(uint32_t* d_states, uint32_t n, const void* d_statics, const uint8_t* d_sd_index,
                        const rsx_controls* d_controls, uint32_t* d_result, uint32_t* d_event_or, uint32_t block, void* stream);
 /* The persistent kernel: `grid` resident blocks pull work items (32 x `granularity` arenas per warp) from a device
@@ -120,8 +122,10 @@ int rsx_sim8_persistent_ex(uint32_t* d_states, uint32_t n, const void* d_statics
  * split 9 with the wheel rays' mesh leaves pooled too (per car, every mesh candidate's leaves evaluated by all threads
  * in one round, the owners replaying them in candidate and walk order); split 11 is split 10 with P3a in one piece;
  * split 14 is split 11 with the 47 feature pairs of the box-triangle SATs that reach them computed by the whole block
- * (up to 18 SATs per round); split 15 is split 14 with the wheel rays' mesh walks run by the whole block level by level
- * (their leaves sorted back into each walk's order; the default: the fastest measured).  Register budget by block: up to 448 threads 144 registers, 512 128.  At
+ * (up to 18 SATs per round); split 15 runs a tick's mesh work in one round each for the wheel rays of both cars and for
+ * every mesh pair of P3b, its BVH walks too by the whole block, level by level (the default: the fastest measured).  Split
+ * 15 launches blocks no larger than their arenas need (256 or 384 threads, at 255 and 168 registers), and a call whose
+ * arenas fit the grid in one round deals them out without the queue.  Register budget of the other sizes: 128.  At
  * most 2^24 arenas and grid 65,535 per call.  Results equal rsx_sim8_multi_raw's whatever grid, block, split or order. */
 #define RSX_LOCKSTEP_MAX_BLOCK 512u
 int rsx_sim8_lockstep_raw(uint32_t* d_states, uint32_t n, const void* d_statics, const uint8_t* d_sd_index,

@@ -26,6 +26,8 @@ RSX_DECL_PERSIST(16)
                                             uint32_t* result, uint32_t* ev_or, const uint32_t* order, uint32_t* counter, uint32_t n,  \
                                             uint32_t width, uint32_t grid, uint32_t block, int split, uint32_t t_first, uint32_t t_last, \
                                             cudaStream_t s);
+RSX_DECL_LOCKSTEP(256)
+RSX_DECL_LOCKSTEP(384)
 RSX_DECL_LOCKSTEP(448)
 RSX_DECL_LOCKSTEP(512)
 cudaError_t rsx_launch_pred_features(const uint32_t* states, const void* sds, const uint8_t* sd_index, const void* controls, uint32_t n,
@@ -56,6 +58,9 @@ cudaError_t rsx_launch_step_tick(uint32_t* buf, const void* sd, uint32_t n, int3
 cudaError_t rsx_launch_sim8_profile(uint32_t* states, const void* sds, const uint8_t* sd_index, const void* controls, uint32_t n,
                                     unsigned long long* prof, cudaStream_t s);
 
+
+constexpr uint32_t kSpreadBlock = 256;  // the lockstep kernel's block and barrier split of the one-launch decisions
+constexpr int kSpreadSplit = 15;        // (the split whose kernels exist in every register budget)
 
 struct rsx_device {
   int ordinal;
@@ -90,6 +95,70 @@ int rsx_set_last_error(int code, const char* msg) {
 // Local memory: the kernels' call chains are known at compile time (no recursion), so the runtime sizes each thread's
 // local memory (about 20 KB: the arena state and the solver's rows) by itself; nothing to configure per device.
 static int configure_current(void) { return RSX_OK; }
+
+// A lockstep launch of n arenas on `grid` blocks of at most `block` threads: the threads to launch per block, the arenas a
+// warp claims at a time, and whether it claims them from the queue.
+struct LockstepPlan {
+  uint32_t block, width;
+  bool queue;
+};
+static LockstepPlan lockstep_plan(uint32_t n, uint32_t grid, uint32_t block, uint32_t split) {
+  const uint64_t lanes = (uint64_t)grid * block;
+  const uint64_t rounds = (n + lanes - 1) / lanes;
+  const uint32_t per = (uint32_t)((n + rounds * grid - 1) / (rounds * grid));  // a block's arenas in one round
+  LockstepPlan p;
+  // Blocks no larger than their arenas need: a scheduler's registers are its warps', and the simulator's inlined phases
+  // spill less in 255 registers (8 warps) or 168 (12) than in 128 (14 and 16).  20,000 arenas (136 per SM): 6.4 ms in 256
+  // threads, 7.5 in 448; 56,000 (379): 10.6 in 384, 11.2 in 448.  Uneven rounds are evened out the same way: 70,001
+  // arenas in two rounds of 256 threads rather than one of 448 and a rest.
+  p.block = block;
+  if (split == kSpreadSplit && per <= 384 && block > 384) p.block = 384;
+  if (split == kSpreadSplit && per <= 256 && block > 256) p.block = 256;
+  // Few arenas a block: one warp per SM until it is full, then more.  A warp's lanes share its instruction fetches, which
+  // bound an SM that runs few warps; spread over more warps the lanes diverge less but each warp fetches for itself.
+  // 2,048 arenas: headline states 3.4 ms in one warp of 14, 3.6 in seven of 2; kickoffs, which hardly diverge, 1.3 and 2.1
+  // ms; 4,096: 4.15 and 1.4 ms in one warp, 4.05 and 1.9 in four.  Up to three arenas get a warp each: 300 arenas 1.8
+  // ms, 2.5 in one warp (kickoffs 1.2 both ways).
+  p.width = per <= 3 ? 1u : per < 32 ? per : 32u;
+  p.queue = rounds > 1;  // one round is dealt out evenly by the kernel (10,007 arenas left 125 of 148 SMs idle: 9.6 ms, now 5.3)
+  return p;
+}
+static cudaError_t lockstep(const LockstepPlan& p, uint32_t* states, const void* sds, const uint8_t* sd_index, const void* controls,
+                            uint32_t* result, uint32_t* ev_or, const uint32_t* order, uint32_t* counter, uint32_t n, uint32_t grid,
+                            int split, uint32_t t0, uint32_t t1, cudaStream_t s) {
+  if (p.queue) {
+    const cudaError_t e = cudaMemsetAsync(counter, 0, 4, s);
+    if (e != cudaSuccess) return e;
+  } else {
+    counter = nullptr;
+  }
+  auto launch = split != kSpreadSplit ? (p.block <= 448 ? rsx_launch_sim8_lockstep_t448 : rsx_launch_sim8_lockstep_t512)
+                : p.block <= 256      ? rsx_launch_sim8_lockstep_t256
+                : p.block <= 384      ? rsx_launch_sim8_lockstep_t384
+                : p.block <= 448      ? rsx_launch_sim8_lockstep_t448
+                                      : rsx_launch_sim8_lockstep_t512;
+  return launch(states, sds, sd_index, controls, result, ev_or, order, counter, n, p.width, grid, p.block, split, t0, t1, s);
+}
+
+// The one-launch decisions (rsx_sim8_raw without a trace, rsx_sim8_multi_raw) by size, on a device of `sms` SMs:
+//   a few arenas (sms / 8): one lane per SM (the plain kernel in blocks of 1), the shortest path of a single arena (1 arena
+//     0.54 ms, 0.60 in the lockstep kernel; 16 arenas 0.80 and 0.81; in one warp 16 take 1.1 - 2.0).
+//   up to `most`: the lockstep kernel in one round.  rsx_sim8_multi_raw, up to 256 arenas per SM: 1,024 arenas 2.5 ms, 6.0 in
+//     warps of 32, kickoffs 1.2 and 1.3; 4,096: 4.1 and 6.9, kickoffs 1.4 both; 32,768: 7.8 and 24.  rsx_sim8_raw, up to one
+//     per SM (37 arenas: 1.2 ms, 1.7 - 2.5 in warps of 32; 148: 1.2 and 3.0, kickoffs 0.89 and 0.98): from there on kickoffs
+//     of one pairing, which neither diverge nor read different StaticData, are faster in few full warps (1,024: 1.00 ms,
+//     1.15 in the lockstep kernel).
+//   above: one thread per arena in the caller's blocks, the reference's shape, which the lockstep kernel's timings at those
+//     sizes are compared with.
+enum class Shape { kLanes, kLockstep, kPlain };
+static cudaError_t one_launch_shape(uint32_t n, uint32_t most_per_sm, uint32_t* sms, Shape* shape) {
+  int dev = 0, count = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, dev);
+  *sms = (uint32_t)count;
+  *shape = n <= *sms / 8 ? Shape::kLanes : n <= *sms * most_per_sm ? Shape::kLockstep : Shape::kPlain;
+  return e;
+}
 
 extern "C" {
 
@@ -198,7 +267,14 @@ int rsx_sim8_raw(uint32_t* d_states, uint32_t n, const void* d_static, const rsx
   if (n == 0) return RSX_OK;
   int c = configure_current();
   if (c != RSX_OK) return c;
-  RSX_CK(rsx_launch_sim8(d_states, d_static, d_controls, d_result, n, d_trace, block, (cudaStream_t)stream));
+  uint32_t sms = 0;
+  Shape shape = Shape::kPlain;
+  if (!d_trace) RSX_CK(one_launch_shape(n, 1, &sms, &shape));
+  if (shape == Shape::kLockstep)
+    RSX_CK(lockstep(lockstep_plan(n, sms, kSpreadBlock, kSpreadSplit), d_states, d_static, nullptr, d_controls, d_result, nullptr,
+                    nullptr, nullptr, n, sms, kSpreadSplit, 1, RSX_TICKS_PER_DECISION, (cudaStream_t)stream));
+  else
+    RSX_CK(rsx_launch_sim8(d_states, d_static, d_controls, d_result, n, d_trace, shape == Shape::kLanes ? 1 : block, (cudaStream_t)stream));
   return RSX_OK;
 }
 
@@ -233,7 +309,15 @@ int rsx_sim8_multi_raw(uint32_t* d_states, uint32_t n, const void* d_statics, co
   if (n == 0) return RSX_OK;
   int c = configure_current();
   if (c != RSX_OK) return c;
-  RSX_CK(rsx_launch_sim8_multi(d_states, d_statics, d_sd_index, d_controls, d_result, d_event_or, n, block, (cudaStream_t)stream));
+  uint32_t sms = 0;
+  Shape shape = Shape::kPlain;
+  RSX_CK(one_launch_shape(n, kSpreadBlock, &sms, &shape));
+  if (shape == Shape::kLockstep)
+    RSX_CK(lockstep(lockstep_plan(n, sms, kSpreadBlock, kSpreadSplit), d_states, d_statics, d_sd_index, d_controls, d_result,
+                    d_event_or, nullptr, nullptr, n, sms, kSpreadSplit, 1, RSX_TICKS_PER_DECISION, (cudaStream_t)stream));
+  else
+    RSX_CK(rsx_launch_sim8_multi(d_states, d_statics, d_sd_index, d_controls, d_result, d_event_or, n,
+                                 shape == Shape::kLanes ? 1 : block, (cudaStream_t)stream));
   return RSX_OK;
 }
 
@@ -290,24 +374,16 @@ int rsx_sim8_lockstep_ex(uint32_t* d_states, uint32_t n, const void* d_statics, 
     return rsx_set_last_error(RSX_E_ARG, "rsx_sim8_lockstep: null buffer, block not a multiple of 32 in 32..512, grid 0 or split not in 0..11, 14, 15");
   if (ticks_per_launch == 0 || RSX_TICKS_PER_DECISION % ticks_per_launch != 0)
     return rsx_set_last_error(RSX_E_ARG, "rsx_sim8_lockstep_ex: ticks_per_launch must divide 8 (1, 2, 4 or 8)");
-  // idle warps claim 32 entries once per tick until their block ends: n plus that overshoot must stay below 2^32
+  // idle warps claim up to 32 entries once per tick until their block ends: n plus that overshoot must stay below 2^32
   if (n > kQueueMaxArenas || grid > kQueueMaxGrid)
     return rsx_set_last_error(RSX_E_ARG, "rsx_sim8_lockstep: at most 16,777,216 arenas and grid 65,535 per call "
                                          "(the 32-bit queue counter must not wrap)");
   if (n == 0) return RSX_OK;
   cudaStream_t s = (cudaStream_t)stream;
-  for (uint32_t t0 = 1; t0 <= RSX_TICKS_PER_DECISION; t0 += ticks_per_launch) {
-    const uint32_t t1 = t0 + ticks_per_launch - 1;
-    RSX_CK(cudaMemsetAsync(d_queue_counter, 0, 4, s));
-    cudaError_t e;
-    if (block <= 448)
-      e = rsx_launch_sim8_lockstep_t448(d_states, d_statics, d_sd_index, d_controls, d_result, d_event_or, d_order, d_queue_counter, n, 32,
-                                        grid, block, (int)split, t0, t1, s);
-    else
-      e = rsx_launch_sim8_lockstep_t512(d_states, d_statics, d_sd_index, d_controls, d_result, d_event_or, d_order, d_queue_counter, n, 32,
-                                        grid, block, (int)split, t0, t1, s);
-    RSX_CK(e);
-  }
+  const LockstepPlan plan = lockstep_plan(n, grid, block, split);
+  for (uint32_t t0 = 1; t0 <= RSX_TICKS_PER_DECISION; t0 += ticks_per_launch)
+    RSX_CK(lockstep(plan, d_states, d_statics, d_sd_index, d_controls, d_result, d_event_or, d_order, d_queue_counter, n, grid, (int)split,
+                    t0, t0 + ticks_per_launch - 1, s));
   return RSX_OK;
 }
 

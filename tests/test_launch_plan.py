@@ -1,0 +1,120 @@
+"""The launch shapes of the decision by size (one lane per SM, the lockstep kernel's register budgets, one round dealt
+out or several from the queue, narrow claims) at the sizes where the shape changes, and the lockstep kernel's lists past
+their capacity: the words, results and events of the persistent kernel without barriers, which steps each arena on one
+lane (every word the same, no tolerance)."""
+import ctypes
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+SMS = 148
+
+
+class Arenas:
+    """n contact-heavy arenas of two car pairings, made on the device, and a reference decision of them."""
+
+    def __init__(self, rsx, dev, n, pairings=2):
+        import torch
+
+        self.t, self.rsx, self.dev, self.n = torch, rsx, dev, n
+        L = self.L = rsx.lib()
+        self.sd = dev.upload_static(np.stack([rsx.build_static(7, p, q) for p, q in [(0, 0), (2, 6)][:pairings]]))
+        self.idx = (torch.arange(n, device=dev.device) % pairings).to(torch.uint8)
+        self.ctl = dev.upload_controls(rsx.random_controls(np.random.default_rng(n), n))
+        self.counter = torch.zeros(1, dtype=torch.int32, device=dev.device)
+        self.ds = dev.alloc_states(n)
+        self.words = rsx.aosoa_words(n)
+        self.start = torch.empty(self.words, dtype=torch.int32, device=dev.device)
+        torch.cuda.synchronize()
+        mix = (ctypes.c_float * 5)(*rsx.MIX_CONTACT_HEAVY)
+        rsx.check(L.rsx_reset_arenas_raw(self.ds.ptr(), n, self.sd.ptr(), self.idx.data_ptr(), 3, mix, None, None, None, dev.stream_ptr()), "reset")
+        self.reference()
+        self.reference()  # the states two decisions in
+        rsx.check(L.rsx_copy_raw(self.start.data_ptr(), self.ds.ptr(), self.words * 4, dev.stream_ptr()), "copy")
+        self.want = self.step(self.reference)
+
+    def outputs(self):
+        self.res = self.t.full((self.n,), -1, dtype=self.t.int32, device=self.dev.device)
+        self.ev = self.t.full((self.n,), -1, dtype=self.t.int32, device=self.dev.device)
+        self.t.cuda.synchronize()
+
+    def reference(self):
+        self.outputs()
+        self.rsx.check(self.L.rsx_sim8_persistent_raw(self.ds.ptr(), self.n, self.sd.ptr(), self.idx.data_ptr(), self.ctl.data_ptr(),
+                                                      self.res.data_ptr(), self.ev.data_ptr(), None, self.counter.data_ptr(), SMS * 4, 64, 1,
+                                                      self.dev.stream_ptr()), "persistent")
+
+    def step(self, f):
+        self.rsx.check(self.L.rsx_copy_raw(self.ds.ptr(), self.start.data_ptr(), self.words * 4, self.dev.stream_ptr()), "copy")
+        self.outputs()
+        f()
+        out = self.t.empty(self.words, dtype=self.t.int32, device=self.dev.device)
+        self.rsx.check(self.L.rsx_copy_raw(out.data_ptr(), self.ds.ptr(), self.words * 4, self.dev.stream_ptr()), "copy")
+        self.dev.sync()
+        return out, self.res.clone(), self.ev.clone()
+
+    def same(self, f, events=True):
+        got = self.step(f)
+        for g, w, name in zip(got, self.want, ("states", "results", "events")):
+            assert (name == "events" and not events) or self.t.equal(g, w), name
+
+    def multi(self, block=32):
+        self.rsx.check(self.L.rsx_sim8_multi_raw(self.ds.ptr(), self.n, self.sd.ptr(), self.idx.data_ptr(), self.ctl.data_ptr(),
+                                                 self.res.data_ptr(), self.ev.data_ptr(), block, self.dev.stream_ptr()), "multi")
+
+    def sim8(self):
+        self.rsx.check(self.L.rsx_sim8_raw(self.ds.ptr(), self.n, self.sd.ptr(), self.ctl.data_ptr(), self.res.data_ptr(), 32, None,
+                                           self.dev.stream_ptr()), "sim8")
+
+    def lockstep(self, grid=SMS, block=448, order=None, ticks=8):
+        self.rsx.check(self.L.rsx_sim8_lockstep_ex(self.ds.ptr(), self.n, self.sd.ptr(), self.idx.data_ptr(), self.ctl.data_ptr(),
+                                                   self.res.data_ptr(), self.ev.data_ptr(), order, self.counter.data_ptr(), grid, block, 15,
+                                                   ticks, self.dev.stream_ptr()), "lockstep")
+
+    def free(self):
+        self.dev.sync()
+        self.ds.free()
+        self.sd.free()
+
+
+@pytest.fixture(scope="module")
+def dev(rsx):
+    d = rsx.SimDevice(0)
+    yield d
+    d.close()
+
+
+# one lane per SM up to SMS / 8; claims of 1 up to 3 arenas a block, then as wide as the block's share, 32 from there; 256
+# threads up to 256 a block
+@pytest.mark.parametrize("n", [1, SMS // 8, SMS // 8 + 1, 3 * SMS, 3 * SMS + 1, 31 * SMS + 5, 32 * SMS + 1, 64 * SMS + 33])
+def test_one_launch_decisions(rsx, dev, n):
+    a = Arenas(rsx, dev, n)
+    a.same(a.multi)
+    a.same(a.lockstep)
+    a.free()
+    b = Arenas(rsx, dev, n, pairings=1)
+    b.same(b.sim8, events=False)  # sim8 writes no events
+    b.free()
+
+
+# the register budgets' edges (256 and 384 arenas a block), one round and two, full blocks whose contact-heavy arenas
+# overflow the mesh lists, a block of one warp
+@pytest.mark.parametrize("n,grid,block", [(256, 1, 448), (257, 1, 448), (384, 1, 448), (385, 1, 448), (448, 1, 448), (449, 1, 448),
+                                          (512, 1, 512), (1345, 3, 448), (2000, 5, 64), (33, 1, 32), (2050, 4, 512)])
+def test_lockstep_blocks(rsx, dev, n, grid, block):
+    a = Arenas(rsx, dev, n)
+    a.same(lambda: a.lockstep(grid, block))
+    perm = a.t.from_numpy(np.random.default_rng(5).permutation(n).astype(np.int32)).to(dev.device)
+    a.same(lambda: a.lockstep(grid, block, perm.data_ptr(), ticks=4))
+    a.free()
+
+
+def test_rounds_and_plain_at_size(rsx, dev):
+    """Two even rounds of the smaller budget, and the plain launch above the lockstep kernel's sizes."""
+    n = SMS * 448 + 77
+    a = Arenas(rsx, dev, n)
+    a.same(a.lockstep)
+    a.same(a.multi)
+    a.free()
