@@ -38,6 +38,51 @@ constexpr uint32_t kBias = kAct + kActBytes, kBiasBytes = (3 * kHid + kOutMma) *
 constexpr uint32_t kMisc = kBias + kBiasBytes;  // mbarrier (8 bytes), TMEM address (4 bytes)
 constexpr uint32_t kSmemBytes = kMisc + 16 + 1024;  // + alignment slack
 
+// Staging a weight matrix W[rows][cols] (row-major, cols a multiple of 8) as a K-major operand, 16 bytes at a time: the
+// eight values of a core-matrix row are eight neighbours of W's row, or of its column where W is staged transposed
+// (element (i, o) = W[o][i]; the threads of a warp then read neighbouring columns).  K is the operand's K extent; what
+// W does not have is zero.  (Value by value, with 2-byte stores, a forward of 65,536 rows took 38.9 us, so 34.8; of
+// 8,192 rows, one tile per CTA, staging is most of it.)
+__device__ __forceinline__ uint4 pack8(const __nv_bfloat16 v[8]) {
+  uint32_t w[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+    w[i] = (uint32_t)__bfloat16_as_ushort(v[2 * i]) | ((uint32_t)__bfloat16_as_ushort(v[2 * i + 1]) << 16);
+  return make_uint4(w[0], w[1], w[2], w[3]);
+}
+// (wide: W is 16-byte aligned)
+__device__ __forceinline__ void stage_rows(unsigned char* dst, const __nv_bfloat16* W, uint32_t rows, uint32_t cols, uint32_t out_rows, uint32_t K,
+                                           bool wide) {
+  const uint32_t chunks = K / 8;
+#pragma unroll 4
+  for (uint32_t i = threadIdx.x; i < out_rows * chunks; i += kRows) {
+    const uint32_t r = i / chunks, k = i % chunks * 8;
+    uint4 v = make_uint4(0u, 0u, 0u, 0u);
+    if (r < rows && k < cols) {
+      const __nv_bfloat16* src = W + (size_t)r * cols + k;
+      if (wide) {
+        v = *reinterpret_cast<const uint4*>(src);
+      } else {
+        __nv_bfloat16 e[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) e[j] = src[j];
+        v = pack8(e);
+      }
+    }
+    *reinterpret_cast<uint4*>(dst + canon(r, k, K)) = v;
+  }
+}
+// element (i, o) = W[o][i] for i < kHid, o < K, zero from out_rows on
+__device__ __forceinline__ void stage_transposed(unsigned char* dst, const __nv_bfloat16* W, uint32_t out_rows, uint32_t K) {
+#pragma unroll 2
+  for (uint32_t o = 0; o < K; o += 8) {
+    __nv_bfloat16 e[8];
+#pragma unroll
+    for (uint32_t j = 0; j < 8; ++j) e[j] = o + j < out_rows ? W[(size_t)(o + j) * kHid + threadIdx.x] : __float2bfloat16_rn(0.0f);
+    *reinterpret_cast<uint4*>(dst + canon(threadIdx.x, o, K)) = pack8(e);
+  }
+}
+
 }  // namespace
 
 extern "C" __global__ void __launch_bounds__(kRows, 1) k_pred_forward_tc(const __nv_bfloat16* __restrict__ wb, const float* __restrict__ wf,
@@ -52,20 +97,12 @@ extern "C" __global__ void __launch_bounds__(kRows, 1) k_pred_forward_tc(const _
   const uint32_t mbar = sbase + kMisc;
 
   // weights and biases into the canonical layout (zero padding: W1's K 48..63, W4's rows 8..15)
-  const __nv_bfloat16 zero = __float2bfloat16_rn(0.0f);
-  for (uint32_t i = tid; i < (uint32_t)(kHid * kInPad); i += kRows) {
-    uint32_t r = i / kInPad, k = i % kInPad;
-    *reinterpret_cast<__nv_bfloat16*>(sm + kW1 + canon(r, k, kInPad)) = k < (uint32_t)kIn ? wb[oW1 + r * kIn + k] : zero;
-  }
-  for (uint32_t i = tid; i < (uint32_t)(kHid * kHid); i += kRows) {
-    uint32_t r = i / kHid, k = i % kHid;
-    *reinterpret_cast<__nv_bfloat16*>(sm + kW2 + canon(r, k, kHid)) = wb[oW2 + i];
-    *reinterpret_cast<__nv_bfloat16*>(sm + kW3 + canon(r, k, kHid)) = wb[oW3 + i];
-  }
-  for (uint32_t i = tid; i < (uint32_t)(kOutMma * kHid); i += kRows) {
-    uint32_t r = i / kHid, k = i % kHid;
-    *reinterpret_cast<__nv_bfloat16*>(sm + kW4 + canon(r, k, kHid)) = r < (uint32_t)kOutPad ? wb[oW4 + r * kHid + k] : zero;
-  }
+  const bool wide = ((uintptr_t)wb & 15u) == 0;  // (the blocks' offsets are multiples of 16 bytes)
+  static_assert(oW1 % 8 == 0 && oW2 % 8 == 0 && oW3 % 8 == 0 && oW4 % 8 == 0, "16-byte offsets");
+  stage_rows(sm + kW1, wb + oW1, kHid, kIn, kHid, kInPad, wide);
+  stage_rows(sm + kW2, wb + oW2, kHid, kHid, kHid, kHid, wide);
+  stage_rows(sm + kW3, wb + oW3, kHid, kHid, kHid, kHid, wide);
+  stage_rows(sm + kW4, wb + oW4, kOutPad, kHid, kOutMma, kHid, wide);
   for (uint32_t i = tid; i < (uint32_t)kHid; i += kRows) {
     bias[i] = wf[ob1 + i];
     bias[kHid + i] = wf[ob2 + i];
@@ -198,16 +235,9 @@ extern "C" __global__ void __launch_bounds__(kRows, 1) k_pred_backward_tc(const 
   const uint32_t tid = threadIdx.x, warp = tid >> 5;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm + bMisc + 8);
   const uint32_t mbar = sbase + bMisc;
-  const __nv_bfloat16 zero = __float2bfloat16_rn(0.0f);
-  for (uint32_t i = tid; i < (uint32_t)(kHid * 16); i += kRows) {  // element (i, o) of W4^T
-    uint32_t r = i / 16, o = i % 16;
-    *reinterpret_cast<__nv_bfloat16*>(sm + bW4T + canon(r, o, 16)) = o < (uint32_t)kOutPad ? wb[oW4 + o * kHid + r] : zero;
-  }
-  for (uint32_t i = tid; i < (uint32_t)(kHid * kHid); i += kRows) {  // W[o][i] -> element (i, o)
-    uint32_t o = i / kHid, r = i % kHid;
-    *reinterpret_cast<__nv_bfloat16*>(sm + bW3T + canon(r, o, kHid)) = wb[oW3 + i];
-    *reinterpret_cast<__nv_bfloat16*>(sm + bW2T + canon(r, o, kHid)) = wb[oW2 + i];
-  }
+  stage_transposed(sm + bW4T, wb + oW4, kOutPad, 16);
+  stage_transposed(sm + bW3T, wb + oW3, kHid, kHid);
+  stage_transposed(sm + bW2T, wb + oW2, kHid, kHid);
   if (tid == 0) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(mbar) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -407,18 +437,30 @@ extern "C" __global__ void __launch_bounds__(kRows) k_pred_wgrad_tc(const __nv_b
   float bias_w4 = 0.0f;   // layer 0: this thread's share of db4[tid % 16]
 #pragma unroll 1
   for (uint32_t c = b_lo; c < b_hi && ok; c += kChunk) {
-    // stage the chunk, transposing: A element (r, b) for r < 128, B element (r, b) for r < N
-    for (uint32_t idx = tid; idx < (uint32_t)kRows * kChunk; idx += kRows) {
-      const uint32_t b = idx / kRows, r = idx % kRows, gb = c + b;
-      __nv_bfloat16 v = gb < b_hi ? asrc[(size_t)gb * kHid + r] : zero;
-      *reinterpret_cast<__nv_bfloat16*>(sm + gA + canon(r, b, kChunk)) = v;
-      if (layer != 0) bias_acc += __bfloat162float(v);
+    // stage the chunk, transposing: A element (r, b) for r < 128, B element (r, b) for r < N; eight batch rows of a
+    // column at a time (neighbouring threads read neighbouring columns; 16-byte stores)
+#pragma unroll 2
+    for (uint32_t b = 0; b < kChunk; b += 8) {
+      __nv_bfloat16 e[8];
+#pragma unroll
+      for (uint32_t j = 0; j < 8; ++j) e[j] = c + b + j < b_hi ? asrc[(size_t)(c + b + j) * kHid + tid] : zero;
+      *reinterpret_cast<uint4*>(sm + gA + canon(tid, b, kChunk)) = pack8(e);
+      if (layer != 0) {
+#pragma unroll
+        for (uint32_t j = 0; j < 8; ++j) bias_acc += __bfloat162float(e[j]);
+      }
     }
-    for (uint32_t idx = tid; idx < N * kChunk; idx += kRows) {
-      const uint32_t b = idx / N, r = idx % N, gb = c + b;
-      __nv_bfloat16 v = (gb < b_hi && r < nb_live) ? bsrc[(size_t)gb * bstride + r] : zero;
-      *reinterpret_cast<__nv_bfloat16*>(sm + gB + canon(r, b, kChunk)) = v;
-      if (layer == 0) bias_w4 += __bfloat162float(v);
+#pragma unroll 2
+    for (uint32_t idx = tid; idx < N * (kChunk / 8); idx += kRows) {
+      const uint32_t r = idx % N, b = idx / N * 8;
+      __nv_bfloat16 e[8];
+#pragma unroll
+      for (uint32_t j = 0; j < 8; ++j) e[j] = c + b + j < b_hi && r < nb_live ? bsrc[(size_t)(c + b + j) * bstride + r] : zero;
+      *reinterpret_cast<uint4*>(sm + gB + canon(r, b, kChunk)) = pack8(e);
+      if (layer == 0) {
+#pragma unroll
+        for (uint32_t j = 0; j < 8; ++j) bias_w4 += __bfloat162float(e[j]);
+      }
     }
     fence_smem_to_async();
     fence_before();
@@ -485,7 +527,10 @@ cudaError_t rsx_launch_pred_wgrads_tc(const void* X, const void* dz, const void*
     if (e != cudaSuccess) return e;
     if (dev >= 0 && dev < 64) configured[dev] = 1;
   }
-  const uint32_t slice = 512, slices = (n + slice - 1) / slice;
+  // Batch rows per CTA: enough CTAs for the chip, few enough partial sums.  A whole training step at 128 / 256 / 512 rows:
+  // batch 2,048 94 / 109 / 135 us, 8,192 114 / 109 / 134, 32,768 224 / 179 / 178 (8,192 took 230 with the operands staged
+  // value by value).
+  const uint32_t slice = n <= 2048 ? 128 : 256, slices = (n + slice - 1) / slice;
   k_pred_wgrad_tc<<<dim3(slices, 4), kRows, kWgradSmemBytes, s>>>((const __nv_bfloat16*)X, (const __nv_bfloat16*)dz, (const __nv_bfloat16*)save,
                                                                   (const __nv_bfloat16*)dsave, n, slice, grad, err);
   return cudaGetLastError();
