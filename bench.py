@@ -63,13 +63,13 @@ def _kc(rd, wr, inst, thr):
 
 
 KERNEL_COUNTERS = {
-    "k_sim8_multi": _kc(5126267136, 5056344576, 1534066674, 10436083984),
-    "k_sim8_lockstep_t448<7>": _kc(6258553856, 5842978816, 1551714381, 10758340571),
-    "k_sim8_lockstep_t512<7>": _kc(6255863552, 5833099776, 1552293325, 10775763619),
-    "k_sim8_lockstep_t448<14>": _kc(5870563840, 5579853312, 1213356967, 11506029617),
-    "k_sim8_lockstep_t512<14>": _kc(5894772480, 5602215168, 1217023574, 11597969422),
-    "k_sim8_lockstep_t448<15>": _kc(5848313600, 5567679232, 1167464173, 11751954768),
-    "k_sim8_lockstep_t512<15>": _kc(5877518848, 5585444608, 1172608364, 11849352609),
+    "k_sim8_multi": _kc(5058114816, 5021709056, 1509326896, 9997320896),
+    "k_sim8_lockstep_t448<7>": _kc(6146897920, 5795379200, 1581091634, 10610346282),
+    "k_sim8_lockstep_t512<7>": _kc(6137490176, 5792792832, 1581875941, 10635629271),
+    "k_sim8_lockstep_t448<14>": _kc(5886416640, 5595306496, 1189371246, 11172830549),
+    "k_sim8_lockstep_t512<14>": _kc(5900027648, 5608007168, 1192384700, 11263047794),
+    "k_sim8_lockstep_t448<15>": _kc(5450868736, 5343553280, 990985466, 11269310229),
+    "k_sim8_lockstep_t512<15>": _kc(5474784256, 5368506112, 992948195, 11330182713),
 }
 
 
