@@ -946,7 +946,8 @@ for _k, _nm in enumerate(["P0", "P1", "P2", "P3a", "P3b", "P4", "P5", "P6", "P7"
 
 LOCKSTEP_ZONE_NAMES = {40: "P0", 41: "P1 pre-tick head (per car)", 42: "P1 wheel rays (per car)", 43: "P1 wheel response (per car)",
                        44: "P2", 45: "P3a", 46: "P3b", 47: "P4", 48: "P5 (3 pieces)", 49: "P6", 29: "P7", 30: "P8 (2 pieces)",
-                       33: "  P3b heads and walks", 34: "  P3b pooled leaf tests", 35: "  P3b additions and tails",
+                       33: "  P3b heads and walks (split 15: job search)", 34: "  P3b pooled leaf tests",
+                       35: "  P3b additions and tails (split 15: heads too)", 36: "  P3b walks over the block (split 15)",
                        60: "copy-in (load_tick)", 61: "copy-out (store_tick)"}
 for _i, _nm in zip([50, 51, 52, 53, 54, 55, 56, 57, 58, 59, 31, 32],
                    ["P0", "P1 head", "P1 rays", "P1 response", "P2", "P3a", "P3b (pool rounds)", "P4", "P5", "P6", "P7", "P8"]):
@@ -998,7 +999,7 @@ def zones(args, dev):
             raise RuntimeError(f"zone run failed ({rc})")
         tot += out.astype(np.float64)
     if args.zones_lockstep:
-        pieces = [40, 41, 42, 43, 44, 45, 46, 47, 48, 49, 29, 30, 33, 34, 35]  # 33-35: P3b's pieces in the pooled splits
+        pieces = [40, 41, 42, 43, 44, 45, 46, 47, 48, 49, 29, 30, 33, 34, 35, 36]  # 33-36: P3b's pieces in the pooled splits
         bars = [50, 51, 52, 53, 54, 55, 56, 57, 58, 59, 31, 32]
     else:
         pieces, bars = [40 + k for k in range(10)], [50 + k for k in range(10)]
