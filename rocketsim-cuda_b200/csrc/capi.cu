@@ -5,6 +5,7 @@
 #include <string.h>
 #include <mutex>
 #include "../../include/rsx.h"
+#include "launch_plan.h"
 #include "state.cuh"
 
 using namespace rsx;
@@ -59,8 +60,7 @@ cudaError_t rsx_launch_sim8_profile(uint32_t* states, const void* sds, const uin
                                     unsigned long long* prof, cudaStream_t s);
 
 
-constexpr uint32_t kSpreadBlock = 256;  // the lockstep kernel's block and barrier split of the one-launch decisions
-constexpr int kSpreadSplit = 15;        // (the split whose kernels exist in every register budget)
+constexpr uint32_t kSpreadBlock = 256;  // the lockstep kernel's block in the one-launch decisions (split kSpreadSplit)
 
 struct rsx_device {
   int ordinal;
@@ -96,33 +96,6 @@ int rsx_set_last_error(int code, const char* msg) {
 // local memory (about 20 KB: the arena state and the solver's rows) by itself; nothing to configure per device.
 static int configure_current(void) { return RSX_OK; }
 
-// A lockstep launch of n arenas on `grid` blocks of at most `block` threads: the threads to launch per block, the arenas a
-// warp claims at a time, and whether it claims them from the queue.
-struct LockstepPlan {
-  uint32_t block, width;
-  bool queue;
-};
-static LockstepPlan lockstep_plan(uint32_t n, uint32_t grid, uint32_t block, uint32_t split) {
-  const uint64_t lanes = (uint64_t)grid * block;
-  const uint64_t rounds = (n + lanes - 1) / lanes;
-  const uint32_t per = (uint32_t)((n + rounds * grid - 1) / (rounds * grid));  // a block's arenas in one round
-  LockstepPlan p;
-  // Blocks no larger than their arenas need: a scheduler's registers are its warps', and the simulator's inlined phases
-  // spill less in 255 registers (8 warps) or 168 (12) than in 128 (14 and 16).  20,000 arenas (136 per SM): 6.4 ms in 256
-  // threads, 7.5 in 448; 56,000 (379): 10.6 in 384, 11.2 in 448.  Uneven rounds are evened out the same way: 70,001
-  // arenas in two rounds of 256 threads rather than one of 448 and a rest.
-  p.block = block;
-  if (split == kSpreadSplit && per <= 384 && block > 384) p.block = 384;
-  if (split == kSpreadSplit && per <= 256 && block > 256) p.block = 256;
-  // Few arenas a block: one warp per SM until it is full, then more.  A warp's lanes share its instruction fetches, which
-  // bound an SM that runs few warps; spread over more warps the lanes diverge less but each warp fetches for itself.
-  // 2,048 arenas: headline states 3.4 ms in one warp of 14, 3.6 in seven of 2; kickoffs, which hardly diverge, 1.3 and 2.1
-  // ms; 4,096: 4.15 and 1.4 ms in one warp, 4.05 and 1.9 in four.  Up to three arenas get a warp each: 300 arenas 1.8
-  // ms, 2.5 in one warp (kickoffs 1.2 both ways).
-  p.width = per <= 3 ? 1u : per < 32 ? per : 32u;
-  p.queue = rounds > 1;  // one round is dealt out evenly by the kernel (10,007 arenas left 125 of 148 SMs idle: 9.6 ms, now 5.3)
-  return p;
-}
 static cudaError_t lockstep(const LockstepPlan& p, uint32_t* states, const void* sds, const uint8_t* sd_index, const void* controls,
                             uint32_t* result, uint32_t* ev_or, const uint32_t* order, uint32_t* counter, uint32_t n, uint32_t grid,
                             int split, uint32_t t0, uint32_t t1, cudaStream_t s) {
@@ -132,7 +105,7 @@ static cudaError_t lockstep(const LockstepPlan& p, uint32_t* states, const void*
   } else {
     counter = nullptr;
   }
-  auto launch = split != kSpreadSplit ? (p.block <= 448 ? rsx_launch_sim8_lockstep_t448 : rsx_launch_sim8_lockstep_t512)
+  auto launch = split != (int)kSpreadSplit ? (p.block <= 448 ? rsx_launch_sim8_lockstep_t448 : rsx_launch_sim8_lockstep_t512)
                 : p.block <= 256      ? rsx_launch_sim8_lockstep_t256
                 : p.block <= 384      ? rsx_launch_sim8_lockstep_t384
                 : p.block <= 448      ? rsx_launch_sim8_lockstep_t448

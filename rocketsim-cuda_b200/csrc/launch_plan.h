@@ -1,0 +1,39 @@
+// The launch shape of a lockstep decision: the threads to launch per block, the arenas a warp claims at a time, and
+// whether it claims them from the queue.  Host code without CUDA calls; capi.cu launches what it says.
+#pragma once
+#include <stdint.h>
+
+namespace rsx {
+
+constexpr uint32_t kSpreadSplit = 15;  // the lockstep split whose kernels exist in every register budget
+
+struct LockstepPlan {
+  uint32_t block, width;
+  bool queue;
+};
+// n arenas on `grid` blocks of at most `block` threads
+inline LockstepPlan lockstep_plan(uint32_t n, uint32_t grid, uint32_t block, uint32_t split) {
+  const uint64_t lanes = (uint64_t)grid * block;
+  const uint64_t rounds = (n + lanes - 1) / lanes;
+  const uint32_t per = (uint32_t)((n + rounds * grid - 1) / (rounds * grid));  // a block's arenas in one round
+  LockstepPlan p;
+  // Blocks no larger than their arenas need: a scheduler's registers are its warps', and the simulator's inlined phases
+  // spill less in 255 registers (8 warps) or 168 (12) than in 128 (14 and 16).  20,000 arenas (136 per SM): 6.4 ms in 256
+  // threads, 7.5 in 448; 56,000 (379): 10.6 in 384, 11.2 in 448.  Uneven rounds are evened out the same way: 70,001
+  // arenas in two rounds of 256 threads rather than one of 448 and a rest.
+  p.block = block;
+  if (split == kSpreadSplit && per <= 384 && block > 384) p.block = 384;
+  if (split == kSpreadSplit && per <= 256 && block > 256) p.block = 256;
+  // Few arenas a block: one warp per SM until it is full, then more.  A warp's lanes share its instruction fetches, which
+  // bound an SM that runs few warps; spread over more warps the lanes diverge less but each warp fetches for itself.
+  // 2,048 arenas: headline states 3.4 ms in one warp of 14, 3.6 in seven of 2; kickoffs, which hardly diverge, 1.3 and 2.1
+  // ms; 4,096: 4.15 and 1.4 ms in one warp, 4.05 and 1.9 in four.  Up to three arenas get a warp each, where the block has
+  // the warps (444 arenas on 148 blocks of one warp, claimed one by one: kickoffs 3.9 ms, in one claim 1.7): 300 arenas
+  // 1.8 ms, 1.9 in one warp (contact-heavy 2.1 both ways; kickoffs 1.3 and 1.1).
+  const uint32_t warps = p.block / 32;
+  p.width = per <= 3 && per <= warps ? 1u : per < 32 ? per : 32u;
+  p.queue = rounds > 1;  // one round is dealt out evenly by the kernel (10,007 arenas left 125 of 148 SMs idle: 9.6 ms, now 5.3)
+  return p;
+}
+
+}  // namespace rsx
