@@ -125,7 +125,8 @@ int rsx_sim8_persistent_ex(uint32_t* d_states, uint32_t n, const void* d_statics
  * (up to 18 SATs per round); split 15 runs a tick's mesh work in one round each for the wheel rays of both cars and for
  * every mesh pair of P3b, its BVH walks too by the whole block, level by level (the default: the fastest measured).  Split
  * 15 launches blocks no larger than their arenas need (256 or 384 threads, at 255 and 168 registers), and a call whose
- * arenas fit the grid in one round deals them out without the queue.  Register budget of the other sizes: 128.  At
+ * arenas fit the grid in one round deals them out without the queue.  Register budget of the other sizes: 128.  Of a
+ * grid past the device's SMs no more blocks are launched than it holds at once or than take the arenas.  At
  * most 2^24 arenas and grid 65,535 per call.  Results equal rsx_sim8_multi_raw's whatever grid, block, split or order. */
 #define RSX_LOCKSTEP_MAX_BLOCK 512u
 int rsx_sim8_lockstep_raw(uint32_t* d_states, uint32_t n, const void* d_statics, const uint8_t* d_sd_index,

@@ -26,7 +26,8 @@ RSX_DECL_PERSIST(16)
   cudaError_t rsx_launch_sim8_lockstep_t##T(uint32_t* states, const void* sds, const uint8_t* sd_index, const void* controls,         \
                                             uint32_t* result, uint32_t* ev_or, const uint32_t* order, uint32_t* counter, uint32_t n,  \
                                             uint32_t width, uint32_t grid, uint32_t block, int split, uint32_t t_first, uint32_t t_last, \
-                                            cudaStream_t s);
+                                            cudaStream_t s);                                                                             \
+  cudaError_t rsx_lockstep_blocks_per_sm_t##T(int split, uint32_t block, int* blocks);
 RSX_DECL_LOCKSTEP(256)
 RSX_DECL_LOCKSTEP(384)
 RSX_DECL_LOCKSTEP(448)
@@ -96,21 +97,43 @@ int rsx_set_last_error(int code, const char* msg) {
 // local memory (about 20 KB: the arena state and the solver's rows) by itself; nothing to configure per device.
 static int configure_current(void) { return RSX_OK; }
 
-static cudaError_t lockstep(const LockstepPlan& p, uint32_t* states, const void* sds, const uint8_t* sd_index, const void* controls,
-                            uint32_t* result, uint32_t* ev_or, const uint32_t* order, uint32_t* counter, uint32_t n, uint32_t grid,
-                            int split, uint32_t t0, uint32_t t1, cudaStream_t s) {
-  if (p.queue) {
-    const cudaError_t e = cudaMemsetAsync(counter, 0, 4, s);
-    if (e != cudaSuccess) return e;
-  } else {
-    counter = nullptr;
+// the lockstep kernel by register budget
+struct LockstepBuild {
+  decltype(&rsx_launch_sim8_lockstep_t448) launch;
+  decltype(&rsx_lockstep_blocks_per_sm_t448) blocks_per_sm;
+};
+static LockstepBuild lockstep_build(uint32_t split, uint32_t block) {
+  if (split == kSpreadSplit && block <= 256) return {rsx_launch_sim8_lockstep_t256, rsx_lockstep_blocks_per_sm_t256};
+  if (split == kSpreadSplit && block <= 384) return {rsx_launch_sim8_lockstep_t384, rsx_lockstep_blocks_per_sm_t384};
+  if (block <= 448) return {rsx_launch_sim8_lockstep_t448, rsx_lockstep_blocks_per_sm_t448};
+  return {rsx_launch_sim8_lockstep_t512, rsx_lockstep_blocks_per_sm_t512};
+}
+static cudaError_t sm_count(uint32_t* sms) {
+  int dev = 0, count = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, dev);
+  *sms = (uint32_t)count;
+  return e;
+}
+// A decision in launches of ticks_per_launch ticks on up to `grid` blocks of up to `block` threads, on a device of `sms` SMs
+static cudaError_t lockstep(uint32_t* states, uint32_t n, const void* sds, const uint8_t* sd_index, const void* controls, uint32_t* result,
+                            uint32_t* ev_or, const uint32_t* order, uint32_t* counter, uint32_t grid, uint32_t block, uint32_t split,
+                            uint32_t ticks_per_launch, uint32_t sms, cudaStream_t s) {
+  cudaError_t e = cudaSuccess;
+  grid = lockstep_grid(n, grid, block, sms, [&] {
+    int blocks = 0;
+    e = lockstep_build(split, block).blocks_per_sm((int)split, block, &blocks);
+    return (uint32_t)blocks;
+  });
+  const LockstepPlan p = lockstep_plan(n, grid, block, split);
+  for (uint32_t t0 = 1; t0 <= RSX_TICKS_PER_DECISION && e == cudaSuccess; t0 += ticks_per_launch) {
+    if (p.queue) e = cudaMemsetAsync(counter, 0, 4, s);
+    if (e == cudaSuccess)
+      e = lockstep_build(split, p.block)
+              .launch(states, sds, sd_index, controls, result, ev_or, order, p.queue ? counter : nullptr, n, p.width, grid, p.block, (int)split,
+                      t0, t0 + ticks_per_launch - 1, s);
   }
-  auto launch = split != (int)kSpreadSplit ? (p.block <= 448 ? rsx_launch_sim8_lockstep_t448 : rsx_launch_sim8_lockstep_t512)
-                : p.block <= 256      ? rsx_launch_sim8_lockstep_t256
-                : p.block <= 384      ? rsx_launch_sim8_lockstep_t384
-                : p.block <= 448      ? rsx_launch_sim8_lockstep_t448
-                                      : rsx_launch_sim8_lockstep_t512;
-  return launch(states, sds, sd_index, controls, result, ev_or, order, counter, n, p.width, grid, p.block, split, t0, t1, s);
+  return e;
 }
 
 // The one-launch decisions (rsx_sim8_raw without a trace, rsx_sim8_multi_raw) by size, on a device of `sms` SMs:
@@ -125,10 +148,7 @@ static cudaError_t lockstep(const LockstepPlan& p, uint32_t* states, const void*
 //     sizes are compared with.
 enum class Shape { kLanes, kLockstep, kPlain };
 static cudaError_t one_launch_shape(uint32_t n, uint32_t most_per_sm, uint32_t* sms, Shape* shape) {
-  int dev = 0, count = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, dev);
-  *sms = (uint32_t)count;
+  const cudaError_t e = sm_count(sms);
   *shape = n <= *sms / 8 ? Shape::kLanes : n <= *sms * most_per_sm ? Shape::kLockstep : Shape::kPlain;
   return e;
 }
@@ -244,8 +264,8 @@ int rsx_sim8_raw(uint32_t* d_states, uint32_t n, const void* d_static, const rsx
   Shape shape = Shape::kPlain;
   if (!d_trace) RSX_CK(one_launch_shape(n, 1, &sms, &shape));
   if (shape == Shape::kLockstep)
-    RSX_CK(lockstep(lockstep_plan(n, sms, kSpreadBlock, kSpreadSplit), d_states, d_static, nullptr, d_controls, d_result, nullptr,
-                    nullptr, nullptr, n, sms, kSpreadSplit, 1, RSX_TICKS_PER_DECISION, (cudaStream_t)stream));
+    RSX_CK(lockstep(d_states, n, d_static, nullptr, d_controls, d_result, nullptr, nullptr, nullptr, sms, kSpreadBlock, kSpreadSplit,
+                    RSX_TICKS_PER_DECISION, sms, (cudaStream_t)stream));
   else
     RSX_CK(rsx_launch_sim8(d_states, d_static, d_controls, d_result, n, d_trace, shape == Shape::kLanes ? 1 : block, (cudaStream_t)stream));
   return RSX_OK;
@@ -286,8 +306,8 @@ int rsx_sim8_multi_raw(uint32_t* d_states, uint32_t n, const void* d_statics, co
   Shape shape = Shape::kPlain;
   RSX_CK(one_launch_shape(n, kSpreadBlock, &sms, &shape));
   if (shape == Shape::kLockstep)
-    RSX_CK(lockstep(lockstep_plan(n, sms, kSpreadBlock, kSpreadSplit), d_states, d_statics, d_sd_index, d_controls, d_result,
-                    d_event_or, nullptr, nullptr, n, sms, kSpreadSplit, 1, RSX_TICKS_PER_DECISION, (cudaStream_t)stream));
+    RSX_CK(lockstep(d_states, n, d_statics, d_sd_index, d_controls, d_result, d_event_or, nullptr, nullptr, sms, kSpreadBlock,
+                    kSpreadSplit, RSX_TICKS_PER_DECISION, sms, (cudaStream_t)stream));
   else
     RSX_CK(rsx_launch_sim8_multi(d_states, d_statics, d_sd_index, d_controls, d_result, d_event_or, n,
                                  shape == Shape::kLanes ? 1 : block, (cudaStream_t)stream));
@@ -352,11 +372,10 @@ int rsx_sim8_lockstep_ex(uint32_t* d_states, uint32_t n, const void* d_statics, 
     return rsx_set_last_error(RSX_E_ARG, "rsx_sim8_lockstep: at most 16,777,216 arenas and grid 65,535 per call "
                                          "(the 32-bit queue counter must not wrap)");
   if (n == 0) return RSX_OK;
-  cudaStream_t s = (cudaStream_t)stream;
-  const LockstepPlan plan = lockstep_plan(n, grid, block, split);
-  for (uint32_t t0 = 1; t0 <= RSX_TICKS_PER_DECISION; t0 += ticks_per_launch)
-    RSX_CK(lockstep(plan, d_states, d_statics, d_sd_index, d_controls, d_result, d_event_or, d_order, d_queue_counter, n, grid, (int)split,
-                    t0, t0 + ticks_per_launch - 1, s));
+  uint32_t sms = 0;
+  RSX_CK(sm_count(&sms));
+  RSX_CK(lockstep(d_states, n, d_statics, d_sd_index, d_controls, d_result, d_event_or, d_order, d_queue_counter, grid, block, split,
+                  ticks_per_launch, sms, (cudaStream_t)stream));
   return RSX_OK;
 }
 

@@ -1111,40 +1111,54 @@ __global__ void __launch_bounds__(RSX_LS_MAXT, 1) K_NAME(uint32_t* states, const
   }
 }
 
+using Kernel = void (*)(uint32_t*, const StaticData*, const uint8_t*, const Controls*, uint32_t*, uint32_t*, const uint32_t*, uint32_t*,
+                        uint32_t, uint32_t, uint32_t, uint32_t);
+static Kernel kernel_of(int split) {
+  switch (split) {
+    case 15: return K_NAME<15>;
+#ifndef RSX_LS_WIDE_REGS
+    case 14: return K_NAME<14>;
+    case 11: return K_NAME<11>;
+    case 10: return K_NAME<10>;
+    case 9: return K_NAME<9>;
+    case 8: return K_NAME<8>;
+    case 7: return K_NAME<7>;
+    case 6: return K_NAME<6>;
+    case 5: return K_NAME<5>;
+    case 4: return K_NAME<4>;
+    case 3: return K_NAME<3>;
+    case 2: return K_NAME<2>;
+    case 1: return K_NAME<1>;
+    case 0: return K_NAME<0>;
+#endif
+    default: return nullptr;
+  }
+}
+static size_t pool_bytes(int split) { return split >= 9 ? sizeof(Pools) : 0; }
+static cudaError_t allow_pool(Kernel k, size_t pool) {
+  return pool ? cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pool) : cudaSuccess;
+}
+
 cudaError_t L_NAME(uint32_t* states, const void* sds, const uint8_t* sd_index, const void* controls, uint32_t* result, uint32_t* ev_or,
                    const uint32_t* order, uint32_t* counter, uint32_t n, uint32_t width, uint32_t grid, uint32_t block, int split,
                    uint32_t t_first, uint32_t t_last, cudaStream_t s) {
-  const StaticData* D = (const StaticData*)sds;
-  const Controls* C = (const Controls*)controls;
-  const size_t pool = split >= 9 ? sizeof(Pools) : 0;
-#define RSX_LS_LAUNCH(k)                                                                                              \
-  if (pool) {                                                                                                         \
-    const cudaError_t e = cudaFuncSetAttribute(K_NAME<k>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pool);    \
-    if (e != cudaSuccess) return e;                                                                                   \
-  }                                                                                                                   \
-  K_NAME<k><<<grid, block, pool, s>>>(states, D, sd_index, C, result, ev_or, order, counter, n, width, t_first, t_last)
-  switch (split) {
-    case 15: RSX_LS_LAUNCH(15); break;
-#ifdef RSX_LS_WIDE_REGS
-    default: return cudaErrorInvalidValue;
-#else
-    case 14: RSX_LS_LAUNCH(14); break;
-    case 11: RSX_LS_LAUNCH(11); break;
-    case 10: RSX_LS_LAUNCH(10); break;
-    case 9: RSX_LS_LAUNCH(9); break;
-    case 8: RSX_LS_LAUNCH(8); break;
-    case 7: RSX_LS_LAUNCH(7); break;
-    case 6: RSX_LS_LAUNCH(6); break;
-    case 5: RSX_LS_LAUNCH(5); break;
-    case 4: RSX_LS_LAUNCH(4); break;
-    case 3: RSX_LS_LAUNCH(3); break;
-    case 2: RSX_LS_LAUNCH(2); break;
-    case 1: RSX_LS_LAUNCH(1); break;
-    default: RSX_LS_LAUNCH(0); break;
-#endif
-  }
-#undef RSX_LS_LAUNCH
+  const Kernel k = kernel_of(split);
+  if (!k) return cudaErrorInvalidValue;
+  const size_t pool = pool_bytes(split);
+  const cudaError_t e = allow_pool(k, pool);
+  if (e != cudaSuccess) return e;
+  k<<<grid, block, pool, s>>>(states, (const StaticData*)sds, sd_index, (const Controls*)controls, result, ev_or, order, counter, n, width,
+                              t_first, t_last);
   return cudaGetLastError();
+}
+
+// how many blocks of `block` threads of the split's kernel one SM of the current device holds at once
+cudaError_t RSX_CAT(rsx_lockstep_blocks_per_sm_t, RSX_LS_MAXT)(int split, uint32_t block, int* blocks) {
+  const Kernel k = kernel_of(split);
+  if (!k) return cudaErrorInvalidValue;
+  const size_t pool = pool_bytes(split);
+  const cudaError_t e = allow_pool(k, pool);
+  return e != cudaSuccess ? e : cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, k, (int)block, pool);
 }
 
 #ifdef RSX_ZONES

@@ -100,10 +100,12 @@ def test_one_launch_decisions(rsx, dev, n):
 
 
 # the register budgets' edges (256 and 384 arenas a block), one round and two, full blocks whose contact-heavy arenas
-# overflow the mesh lists, a block of one warp, up to three arenas a block in fewer warps than that
+# overflow the mesh lists, a block of one warp, up to three arenas a block in fewer warps than that, more blocks than the
+# device holds at once (one round and several, both register budgets)
 @pytest.mark.parametrize("n,grid,block", [(256, 1, 448), (257, 1, 448), (384, 1, 448), (385, 1, 448), (448, 1, 448), (449, 1, 448),
                                           (512, 1, 512), (1345, 3, 448), (2000, 5, 64), (33, 1, 32), (2050, 4, 512),
-                                          (444, 148, 32), (444, 148, 64)])
+                                          (444, 148, 32), (444, 148, 64), (4096, 1480, 64), (600, 296, 224),
+                                          (40001, 296, 224), (40001, 1480, 64)])
 def test_lockstep_blocks(rsx, dev, n, grid, block):
     a = Arenas(rsx, dev, n)
     a.same(lambda: a.lockstep(grid, block))

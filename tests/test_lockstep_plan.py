@@ -1,6 +1,7 @@
-"""The lockstep decision's launch plan (csrc/launch_plan.h), on the CPU: for every size, grid and block the claims cover
-the arenas, and a call whose arenas fit the grid in one round gives no warp a second claim (a warp steps its claims one
-after another, a whole decision each)."""
+"""The lockstep decision's launch plan (csrc/launch_plan.h), on the CPU, over sizes, grids and blocks: a call whose arenas
+fit the grid in one round gives no warp a second claim (a warp steps its claims one after another, a whole decision each),
+and a grid past the SMs is launched with no more blocks than the device holds at once and, below that, no more than hold
+the arenas."""
 import os
 import shutil
 import subprocess
@@ -34,13 +35,28 @@ int main() {
           if (one) ok = ok && (claims + grid - 1) / grid <= p.block / 32;  // the blocks' shares differ by one claim at most
           if (!ok && bad++ < 5) std::printf("n %u grid %u block %u split %u: block %u width %u queue %d\n", n, grid, block, split, p.block, p.width, p.queue);
         }
-  std::printf("plans %ld one-round %ld narrow %ld bad %ld\n", plans, one_round, narrow, bad);
+  // the grid on 148 SMs that hold `held` blocks each
+  long capped = 0;
+  for (uint32_t grid : {1u, 37u, 148u, 149u, 296u, 592u, 1480u, 65535u})
+    for (uint32_t block = 32; block <= 512; block += 32)
+      for (uint32_t held = 1; held <= 8; ++held)
+        for (uint64_t k = 1; k <= 400000; k += 1 + k / 10) {
+          const uint32_t n = (uint32_t)k, got = lockstep_grid(n, grid, block, 148, [&] { return held; });
+          const uint64_t full = 148u * held, lanes = (uint64_t)got * block;
+          ++plans;
+          capped += got < grid;
+          bool ok = got >= 1 && got <= grid && (grid <= 148 ? got == grid : got <= full);
+          // fewer blocks than asked for: as many as the device holds, or as many as take the arenas in one round and no SM's worth more
+          if (got < grid) ok = ok && got % 148 == 0 && (got == full || (lanes >= n && (got == 148 || lanes - 148ull * block < n)));
+          if (!ok && bad++ < 5) std::printf("n %u grid %u block %u held %u: grid %u\n", n, grid, block, held, got);
+        }
+  std::printf("plans %ld one-round %ld narrow %ld capped %ld bad %ld\n", plans, one_round, narrow, capped, bad);
   return bad != 0;
 }
 """
 
 
-def test_one_round_gives_no_warp_two_claims(tmp_path):
+def test_plan(tmp_path):
     if shutil.which("g++") is None:
         pytest.skip("no C++ compiler")
     src, exe = tmp_path / "plan.cpp", tmp_path / "plan"
@@ -49,5 +65,5 @@ def test_one_round_gives_no_warp_two_claims(tmp_path):
     out = subprocess.run([str(exe)], capture_output=True, text=True, timeout=300)
     assert out.returncode == 0, out.stdout
     words = out.stdout.split()
-    for name in ("one-round", "narrow"):
+    for name in ("one-round", "narrow", "capped"):
         assert int(words[words.index(name) + 1]) > 1000, out.stdout
