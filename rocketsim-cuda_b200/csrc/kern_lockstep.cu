@@ -50,6 +50,10 @@
     RSX_ZONE_END(zb_, id);   \
   } while (0)
 #define L_NAME RSX_CAT(rsx_launch_sim8_lockstep_t, RSX_LS_MAXT)
+// Counters of the test build (lists_check.cu; empty otherwise): how often split 15's ways past a full list are taken
+#ifndef LS_COUNT
+#define LS_COUNT(which)
+#endif
 
 namespace {
 // ---- split 9: P3b with the leaf tests of every arena of the block pooled ----
@@ -99,10 +103,11 @@ struct RayPoolSmem {
 // split 15: mesh walks by the whole block.  Jobs (a body's query box against a mesh body) are listed in shared memory,
 // the block walks all their BVHs level by level (front: the nodes of one level with their path keys, sim/ray.cuh
 // walk_expand), and the leaves found are put in each job's stack-walk order by a counting sort by job and a ranking by
-// key within the job.  A job that loses a node or a leaf to a full list, or whose tree is deeper than the keys hold, is
-// marked and done by its own lane; the other jobs are whole.
+// key within the job.  A job that loses a node, a leaf or a hit to a full list, or whose tree is deeper than the keys hold,
+// is marked and done by its own lane (in P3b it is tried again first); the other jobs are whole.
 constexpr uint32_t kJobMask = 511u, kHeadMask = 8191u;
 constexpr int kJobBits = 9, kHeadBits = 13;  // job, then mesh (4 bits), then node or leaf
+constexpr uint32_t kLostFull = 1u, kLostDeep = 2u;  // marks of lost[]
 template <int JOBS, int FRONT, int LEAVES>
 struct WalkLists {
   uint32_t cnt[JOBS], seg[JOBS], fill[JOBS], lost[JOBS];
@@ -113,7 +118,19 @@ struct WalkLists {
   uint16_t byjob[LEAVES];       // the entries above, by job
   uint32_t njobs, nfront[sim::kWalkLevels + 1], nleaf;
 };
+#ifndef RSX_LS_SMALL_LISTS
 constexpr int kWalkRayJobs = 144, kWalkRayFront = 384, kWalkRayLeaves = 400;
+constexpr int kWalkPairJobs = 208, kWalkPairFront = 640, kWalkPairLeaves = 704;
+constexpr int kWalkHits = 128;
+constexpr int kWalkSats = 48;      // SATs of a round whose feature pairs the block computes, kWalkFeat at a time
+constexpr int kWalkFeat = 15;
+#else  // the test build: a few contact-heavy arenas fill every list
+constexpr int kWalkRayJobs = 16, kWalkRayFront = 24, kWalkRayLeaves = 24;
+constexpr int kWalkPairJobs = 24, kWalkPairFront = 32, kWalkPairLeaves = 32;
+constexpr int kWalkHits = 4;
+constexpr int kWalkSats = 2;
+constexpr int kWalkFeat = 1;
+#endif
 constexpr int kWalkRayLane = 8;  // jobs of one lane (both cars)
 struct RayWalkSmem {
   sim::RayMeshJob job[kWalkRayJobs];
@@ -123,12 +140,8 @@ struct RayWalkSmem {
   sim::RayLeaf out[kWalkRayLeaves];
   uint32_t at[kWalkRayLeaves];  // mesh | leaf << 4 of out[]
 };
-constexpr int kWalkPairJobs = 208, kWalkPairFront = 640, kWalkPairLeaves = 704;
 constexpr int kWalkPairLane = 8;   // jobs of one lane in one round
 constexpr int kWalkPairRounds = 3; // from this round on a job the lists lost is done by its lane alone
-constexpr int kWalkHits = 128;
-constexpr int kWalkSats = 48;      // SATs of a round whose feature pairs the block computes, kWalkFeat at a time
-constexpr int kWalkFeat = 15;
 struct PairJob {                   // a sim::LeafJob without what the static data holds
   uint8_t kind, mesh, body;
   union {
@@ -153,6 +166,7 @@ struct PairWalkSmem {
 };
 static_assert(sizeof(sim::FeatPair) * kWalkFeat * sim::kPairs <= sizeof(PairJob) * kWalkPairJobs, "the feature pairs fit over the jobs");
 static_assert(sizeof(RayWalkSmem) + 256 <= 63 * 1024 && sizeof(PairWalkSmem) + 256 <= 63 * 1024, "a 64 KB carveout");
+static_assert(kWalkPairFront >= kWalkPairJobs, "every job starts as an entry of the first level");
 static_assert(kWalkPairJobs <= 512 && kWalkRayJobs <= 512 && kMeshes <= 16 && kWalkPairLeaves < 65536 && kMaxTris < 65536 &&
                   kWalkHits < 65535 && kMaxNodes < (1 << 19) && kMaxLeaves < (1 << 19),
               "the lists' fields hold their values");
@@ -422,6 +436,11 @@ __device__ __noinline__ void rays_pooled(ArenaState& s, const StaticData* D, boo
   RSX_ZONE_END(zr5, 8);
 }
 
+template <class Lists>
+__device__ __forceinline__ void mark_lost(Lists& w, uint32_t q, uint32_t why) {
+  atomicOr(&w.lost[q], why);
+  LS_COUNT(why == kLostDeep ? kCountDeep : kCountFull);
+}
 // The levels of a walk and the order of its leaves (split 15; every thread of the block calls it, after a barrier behind
 // the jobs' writes).  box(q): job q's box; expand(item, key, level, emit): the children of a front item whose boxes meet
 // the job's; keep(entry): whether a leaf entry is kept.  Afterwards each kept leaf's entry is in byjob[seg[q] ..
@@ -444,17 +463,17 @@ __device__ __forceinline__ void walk_levels(WalkLists<JOBS, FRONT, LEAVES>& w, E
             w.key[e] = (uint16_t)key;
             atomicAdd(&w.cnt[q], 1u);
           } else {
-            w.lost[q] = 1;
+            mark_lost(w, q, kLostFull);
           }
         } else if (level + 1 == sim::kWalkLevels) {
-          w.lost[q] = 1;
+          mark_lost(w, q, kLostDeep);
         } else {
           const uint32_t f = atomicAdd(&w.nfront[level + 1], 1u);
           if (f < (uint32_t)FRONT) {
             w.front[cur ^ 1][f] = head | (ch << kHeadBits);
             w.fkey[cur ^ 1][f] = (uint16_t)key;
           } else {
-            w.lost[q] = 1;
+            mark_lost(w, q, kLostFull);
           }
         }
       });
@@ -559,7 +578,7 @@ __device__ __noinline__ void rays_walk_both(ArenaState& s, const StaticData* sds
           sm.w.front[0][f] = q | ((uint32_t)m << kJobBits);
           sm.w.fkey[0][f] = (uint16_t)sim::walk_root_key(m);
         } else {
-          sm.w.lost[q] = 1;
+          mark_lost(sm.w, q, kLostFull);
         }
       }
     }
@@ -607,6 +626,7 @@ __device__ __noinline__ void rays_walk_both(ArenaState& s, const StaticData* sds
           }
           continue;
         }
+        LS_COUNT(kCountRayAlone);
       }
       sim::ray_body(s, *D, w, &pk[ci]);
     }
@@ -727,7 +747,7 @@ __device__ __noinline__ void p3b_walk_all(ArenaState& s, const StaticData* sds, 
         if (h.found) {
           i = atomicAdd(&sm.nhit, 1u) + 1;
           if (i <= (uint32_t)kWalkHits) sm.hit[i - 1] = h;
-          else sm.w.lost[q] = 1;
+          else mark_lost(sm.w, q, kLostFull);
         }
         sm.at_hit[at] = (uint16_t)(i <= (uint32_t)kWalkHits ? i : 0u);
       };
@@ -748,6 +768,7 @@ __device__ __noinline__ void p3b_walk_all(ArenaState& s, const StaticData* sds, 
             sm.front_at[d] = at | (q << 16);
             continue;
           }
+          LS_COUNT(kCountSat);
           sim::FeatPair P[sim::kPairs];  // past the list: this thread computes them itself
           sim::enum_pairs(f.hu, f.q, f.e, P);
           sim::leaf_test_back(f, P, &h);
@@ -797,8 +818,10 @@ __device__ __noinline__ void p3b_walk_all(ArenaState& s, const StaticData* sds, 
           L.walk_done = true;
           sim::p3b_close(s, *D, L);
         } else if (has && round >= kWalkPairRounds) {
+          LS_COUNT(kCountAlone);
           sim::p3b_job_alone(s, *D, L);
         } else {  // its job found no room: the next round
+          LS_COUNT(kCountWait);
           more = true;
           break;
         }

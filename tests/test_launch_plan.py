@@ -1,8 +1,9 @@
 """The launch shapes of the decision by size (one lane per SM, the lockstep kernel's register budgets, one round dealt
-out or several from the queue, narrow claims) at the sizes where the shape changes, and the lockstep kernel's lists past
-their capacity: the words, results and events of the persistent kernel without barriers, which steps each arena on one
-lane (every word the same, no tolerance)."""
+out or several from the queue, narrow claims) at the sizes where the shape changes, the lockstep kernel's lists past their
+capacity: the words, results and events of the persistent kernel without barriers,
+which steps each arena on one lane (every word the same, no tolerance)."""
 import ctypes
+import os
 
 import numpy as np
 import pytest
@@ -99,8 +100,8 @@ def test_one_launch_decisions(rsx, dev, n):
     b.free()
 
 
-# the register budgets' edges (256 and 384 arenas a block), one round and two, full blocks whose contact-heavy arenas
-# overflow the mesh lists, a block of one warp, up to three arenas a block in fewer warps than that, more blocks than the
+# the register budgets' edges (256 and 384 arenas a block), one round and two, full blocks of contact-heavy arenas (more mesh
+# jobs than the lists hold), a block of one warp, up to three arenas a block in fewer warps than that, more blocks than the
 # device holds at once (one round and several, both register budgets)
 @pytest.mark.parametrize("n,grid,block", [(256, 1, 448), (257, 1, 448), (384, 1, 448), (385, 1, 448), (448, 1, 448), (449, 1, 448),
                                           (512, 1, 512), (1345, 3, 448), (2000, 5, 64), (33, 1, 32), (2050, 4, 512),
@@ -121,3 +122,32 @@ def test_rounds_and_plain_at_size(rsx, dev):
     a.same(a.lockstep)
     a.same(a.multi)
     a.free()
+
+
+# ---- split 15's mesh lists, in the build with short lists and counters (csrc/lists_check.cu) ----
+COUNTS = ("full", "deep", "alone", "wait", "sat", "ray_alone")
+
+
+@pytest.fixture(scope="module")
+def lists(rsx):
+    lib = ctypes.CDLL(os.path.join(os.path.dirname(rsx.LIB_PATH), "librsx_lists.so"))
+    vp, u32 = ctypes.c_void_p, ctypes.c_uint32
+    lib.rsx_lists_decide.argtypes = [vp, u32, vp, vp, vp, vp, vp, u32, u32, u32, vp, vp]
+    return lib
+
+
+def decide_counted(lists, a, width, grid, block, counts):
+    c = (ctypes.c_uint32 * len(COUNTS))()
+    rc = lists.rsx_lists_decide(a.ds.ptr(), a.n, a.sd.ptr(), a.idx.data_ptr(), a.ctl.data_ptr(), a.res.data_ptr(), a.ev.data_ptr(), width, grid,
+                                block, c, a.dev.stream_ptr())
+    assert rc == 0
+    counts.update(zip(COUNTS, c))
+
+
+@pytest.mark.parametrize("n,grid,block", [(448, 1, 448), (200, 1, 224), (900, 4, 256)])
+def test_every_way_past_a_full_list(rsx, dev, lists, n, grid, block):
+    a, counts = Arenas(rsx, dev, n), {}
+    a.same(lambda: decide_counted(lists, a, 32, grid, block, counts))
+    assert counts["deep"] == 0 and all(counts[k] > 0 for k in COUNTS if k != "deep"), counts
+    a.free()
+
