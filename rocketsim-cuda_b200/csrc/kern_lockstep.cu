@@ -104,7 +104,7 @@ struct RayPoolSmem {
 // the block walks all their BVHs level by level (front: the nodes of one level with their path keys, sim/ray.cuh
 // walk_expand), and the leaves found are put in each job's stack-walk order by a counting sort by job and a ranking by
 // key within the job.  A job that loses a node, a leaf or a hit to a full list, or whose tree is deeper than the keys hold,
-// is marked and done by its own lane (in P3b it is tried again first); the other jobs are whole.
+// is marked and done by its own lane (in P3b a full list is tried again first); the other jobs are whole.
 constexpr uint32_t kJobMask = 511u, kHeadMask = 8191u;
 constexpr int kJobBits = 9, kHeadBits = 13;  // job, then mesh (4 bits), then node or leaf
 constexpr uint32_t kLostFull = 1u, kLostDeep = 2u;  // marks of lost[]
@@ -141,7 +141,7 @@ struct RayWalkSmem {
   uint32_t at[kWalkRayLeaves];  // mesh | leaf << 4 of out[]
 };
 constexpr int kWalkPairLane = 8;   // jobs of one lane in one round
-constexpr int kWalkPairRounds = 3; // from this round on a job the lists lost is done by its lane alone
+constexpr int kWalkPairRounds = 3; // from this round on a job lost to a full list is done by its lane alone
 struct PairJob {                   // a sim::LeafJob without what the static data holds
   uint8_t kind, mesh, body;
   union {
@@ -817,7 +817,7 @@ __device__ __noinline__ void p3b_walk_all(ArenaState& s, const StaticData* sds, 
           }
           L.walk_done = true;
           sim::p3b_close(s, *D, L);
-        } else if (has && round >= kWalkPairRounds) {
+        } else if (has && (round >= kWalkPairRounds || (sm.w.lost[jslot[j] & kJobMask] & kLostDeep))) {  // (no round holds a deep tree)
           LS_COUNT(kCountAlone);
           sim::p3b_job_alone(s, *D, L);
         } else {  // its job found no room: the next round

@@ -1,6 +1,6 @@
 """The launch shapes of the decision by size (one lane per SM, the lockstep kernel's register budgets, one round dealt
 out or several from the queue, narrow claims) at the sizes where the shape changes, the lockstep kernel's lists past their
-capacity: the words, results and events of the persistent kernel without barriers,
+capacity and trees deeper than its walks hold: the words, results and events of the persistent kernel without barriers,
 which steps each arena on one lane (every word the same, no tolerance)."""
 import ctypes
 import os
@@ -16,12 +16,17 @@ SMS = 148
 class Arenas:
     """n contact-heavy arenas of two car pairings, made on the device, and a reference decision of them."""
 
-    def __init__(self, rsx, dev, n, pairings=2):
+    def __init__(self, rsx, dev, n, pairings=2, change=None):
+        """change: applied to each pairing's StaticData words."""
         import torch
 
         self.t, self.rsx, self.dev, self.n = torch, rsx, dev, n
         L = self.L = rsx.lib()
-        self.sd = dev.upload_static(np.stack([rsx.build_static(7, p, q) for p, q in [(0, 0), (2, 6)][:pairings]]))
+        statics = np.stack([rsx.build_static(7, p, q) for p, q in [(0, 0), (2, 6)][:pairings]])
+        if change:
+            for words in statics:
+                change(words)
+        self.sd = dev.upload_static(statics)
         self.idx = (torch.arange(n, device=dev.device) % pairings).to(torch.uint8)
         self.ctl = dev.upload_controls(rsx.random_controls(np.random.default_rng(n), n))
         self.counter = torch.zeros(1, dtype=torch.int32, device=dev.device)
@@ -133,6 +138,7 @@ def lists(rsx):
     lib = ctypes.CDLL(os.path.join(os.path.dirname(rsx.LIB_PATH), "librsx_lists.so"))
     vp, u32 = ctypes.c_void_p, ctypes.c_uint32
     lib.rsx_lists_decide.argtypes = [vp, u32, vp, vp, vp, vp, vp, u32, u32, u32, vp, vp]
+    lib.rsx_lists_deepen.argtypes = [vp, u32]
     return lib
 
 
@@ -151,3 +157,23 @@ def test_every_way_past_a_full_list(rsx, dev, lists, n, grid, block):
     assert counts["deep"] == 0 and all(counts[k] > 0 for k in COUNTS if k != "deep"), counts
     a.free()
 
+
+# the worlds' trees have five levels and the keys hold six: one more, the first that is too deep, and a chain that every walk
+# leaves before it reaches the tree.  One arena a block: no list is full, so a deep job is its lane's in the round that finds it
+@pytest.mark.parametrize("levels", [1, 2, 6])
+def test_trees_deeper_than_the_keys(rsx, dev, lists, levels):
+    def deepen(words):
+        assert lists.rsx_lists_deepen(words.ctypes.data, levels) == 0
+
+    n, counts = 96, {}
+    plain, a = Arenas(rsx, dev, n), Arenas(rsx, dev, n, change=deepen)
+    for deep, flat, name in zip(a.want, plain.want, ("states", "results", "events")):
+        assert a.t.equal(deep, flat), name  # the walks reach the same leaves
+    a.same(lambda: decide_counted(lists, a, 1, n, 32, counts))
+    assert (counts["deep"] > 0) == (levels > 1), counts
+    if levels == 6:
+        assert counts["full"] == 0 and counts["wait"] == 0 and counts["alone"] > 0 and counts["ray_alone"] > 0, counts
+    for block in (32, 256):  # the library's kernel
+        a.same(lambda: a.lockstep(n, block))
+    a.free()
+    plain.free()
