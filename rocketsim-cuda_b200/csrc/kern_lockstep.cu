@@ -848,34 +848,47 @@ __global__ void __launch_bounds__(RSX_LS_MAXT, 1) K_NAME(uint32_t* states, const
   Controls c0, c1;
   const StaticData* D = sds;
   uint32_t a = 0, di = 0, t = 0, scored = 0, unimpl = 0, ev = 0;
-  // without a queue the claims are dealt out evenly: over the identity order each block's in a row (neighbouring arenas on
-  // one SM: 2% faster at 65,536 arenas than the blocks in turn), over another order the blocks in turn (its costliest
-  // arenas come first)
+  // without a queue the claims are dealt out evenly: split 15 over the identity order each block's in a row (neighbouring
+  // arenas on one SM: 2% faster at 65,536 arenas than the blocks in turn; the splits below 9 are up to 9% slower so), else
+  // the blocks in turn (another order's costliest arenas come first)
+  const bool rows = SPLIT >= 15 && !order;
   const uint32_t nw = blockDim.x >> 5, warp = threadIdx.x >> 5, claims = (n + width - 1) / width;
-  const uint32_t first = order ? blockIdx.x : (uint32_t)((uint64_t)claims * blockIdx.x / gridDim.x), step = order ? gridDim.x : 1u;
-  const uint32_t end = order ? claims : (uint32_t)((uint64_t)claims * (blockIdx.x + 1) / gridDim.x);
+  const uint32_t first = rows ? (uint32_t)((uint64_t)claims * blockIdx.x / gridDim.x) : blockIdx.x, step = rows ? 1u : gridDim.x;
+  const uint32_t end = rows ? (uint32_t)((uint64_t)claims * (blockIdx.x + 1) / gridDim.x) : claims;
   uint32_t next = first + warp * step;
   bool busy = false;               // the warp holds a claim (uniform over the warp)
-  bool have = false, ovf = false;  // the lane steps an arena
+  bool have = false, live = false, ovf = false;  // the lane steps an arena, which is its own
   for (;;) {
     // a warp without arenas claims its next ones
     if (!busy) {
       uint32_t base = 0;
-      if (counter) {
-        if (lane == 0) base = atomicAdd(counter, width);
-        base = __shfl_sync(0xFFFFFFFFu, base, 0);
-      } else {
-        base = next < end ? next * width : n;
-        next += nw * step;
+      if (lane == 0) {
+        if (counter) {
+          base = atomicAdd(counter, width);
+        } else {
+          base = next < end ? next * width : n;
+          next += nw * step;
+        }
       }
+      base = __shfl_sync(0xFFFFFFFFu, base, 0);
       if (base < n) {
         busy = true;
         t = t_first;
+        // A lane past the claim's arenas, or at an order entry past n (not a permutation): where the block pools its work it
+        // steps nothing (a copy's jobs would fill the pools); else it steps a copy of its warp's first arena and stores
+        // nothing, so that the branches on `have` are uniform over a warp, for the compiler too (65,536 arenas, splits 1 and
+        // 7: 3 - 4% faster).
         const uint32_t i = base + lane;
         a = lane < width && i < n ? (order ? order[i] : i) : n;
-        // (a lane past the claim's arenas, or at an order entry past n (not a permutation), steps nothing)
-        if (a < n) {
-          have = true;
+        live = a < n;
+        have = live;
+        if (SPLIT < 9) {
+          const uint32_t own = __ballot_sync(0xFFFFFFFFu, live);
+          const uint32_t first_a = __shfl_sync(0xFFFFFFFFu, a, __ffs(own) - 1);
+          if (!live) a = first_a;
+          have = own != 0;
+        }
+        if (have) {
           di = sd_index ? sd_index[a] : 0;
           D = sds + di;
           RSX_ZONE_BEGIN(zl);
@@ -889,7 +902,10 @@ __global__ void __launch_bounds__(RSX_LS_MAXT, 1) K_NAME(uint32_t* states, const
             scored = r0 & kScoredMask;
             unimpl = r0 & kUnimplemented;
             ev = ev_or ? ev_or[a] : 0u;
-            if (scored) have = false;  // decided in an earlier launch: the buffer holds its goal state
+            if (scored) {  // decided in an earlier launch: the buffer holds its goal state
+              live = false;
+              if (SPLIT >= 9) have = false;
+            }
           }
           ovf = false;
         }
@@ -1115,19 +1131,21 @@ __global__ void __launch_bounds__(RSX_LS_MAXT, 1) K_NAME(uint32_t* states, const
         ev |= s.events;
         if (sim::ball_scored(s, *D)) {
           scored = t;
-          store_tick(states, a, &s);
+          if (live) store_tick(states, a, &s);
           ovf = sim::any_overflow(s);
         }
       }
       if (t == t_last) {  // the end of this launch's ticks (tick 8: of the decision)
         RSX_ZONE_BEGIN(zs);
         if (scored == 0) {
-          store_tick(states, a, &s);
+          if (live) store_tick(states, a, &s);
           ovf = sim::any_overflow(s);
         }
         RSX_ZONE_END(zs, 61);
-        if (ev_or) ev_or[a] = ev;
-        result[a] = scored | unimpl | (ovf ? kOverflow : 0u);
+        if (live) {
+          if (ev_or) ev_or[a] = ev;
+          result[a] = scored | unimpl | (ovf ? kOverflow : 0u);
+        }
       }
     }
     if (busy && t++ == t_last) busy = have = false;
