@@ -73,16 +73,9 @@ KERNEL_COUNTERS = {
 }
 
 
-def kernel_name(config):
-    m = config["mode"]
-    if m == "plain":
-        return "k_sim8_multi"
-    if m == "sim8":
-        return "k_sim8"
-    if m == "persistent":
-        return f"k_sim8_persistent_b{config['min_blocks']}"
-    t = 448 if config["block"] <= 448 else 512
-    name = f"k_sim8_lockstep_t{t}<{config['split']}>"
+def kernel_name(run, config):
+    """The kernel that the runner's decision launches for this configuration at its size."""
+    name = run.kernel(config)
     return name if config.get("ticks", 8) == 8 else f"{name} x{8 // config['ticks']} launches"
 
 
@@ -539,7 +532,7 @@ def run_ours(args):
         res_all, ev_all = leg.record_decisions(config, args.steps)
         step_path_same = bool(torch.equal(run.snapshot(), words_tuned))  # the step-by-step replay ends where the graphs did
         vs_oracle = oracle_compare(L, sds, idx, st, leg.ctl_host, np.arange(n), leg.words_of(words_tuned), res_all, ev_all)
-        vs_oracle["config"] = kernel_name(config)
+        vs_oracle["config"] = kernel_name(run, config)
         vs_oracle["graph_and_step_paths_equal"] = step_path_same
 
     # ---- recall / precision of the predictor on the timed decisions ----
@@ -610,7 +603,7 @@ def run_ours(args):
         pass
     peak = float(peaks.get("hbm_gbs", 6650.0))
     achieved = alg_bytes / (mean_ms / 1e3) / 1e9
-    kname = kernel_name(config)
+    kname = kernel_name(run, config)
     kc = KERNEL_COUNTERS.get(kname)
     roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                 "traffic": kc["dram_bytes_per_arena"] * n if kc else None,
@@ -710,7 +703,7 @@ def one_pairing_leg(args, dev, config, pred):
     cfg = dict(config)
     t, _ = leg.timed(cfg, graph=not args.no_graph and cfg["mode"] != "plain")
     out["tuned"] = args.arenas * 8 * args.steps / (t / 1e3)
-    out["tuned_config"] = kernel_name(cfg)
+    out["tuned_config"] = kernel_name(leg.run, cfg)
     out["same_words"] = bool(leg.torch.equal(leg.run.snapshot(), w_sim8))
     del w_sim8
     leg.free()
@@ -744,7 +737,7 @@ def large_leg(args, dev, pred, L):
             out["lockstep_unbinned"] = n * 8 * a2.steps / (t_unb / 1e3)
     t_ms, _ = leg.timed(config, graph=graph)
     out["tuned"] = n * 8 * a2.steps / (t_ms / 1e3)
-    out["tuned_config"] = {"kernel": kernel_name(config), **config}
+    out["tuned_config"] = {"kernel": kernel_name(leg.run, config), **config}
     out["speedup_vs_plain"] = out["tuned"] / out["plain"]
     words = leg.run.snapshot()
     out["bit_exact_vs_plain"] = bool(torch.equal(words, w_plain))
@@ -781,17 +774,19 @@ def profile_variants(args, leg):
             run.step(leg.dctl[(8 + s) % leg.steps].data_ptr(), cfg)
         e1.record(run.stream)
         e1.synchronize()
-        out.append({"kernel": kernel_name(cfg), "ms": e0.elapsed_time(e1)})
+        out.append({"kernel": kernel_name(run, cfg), "ms": e0.elapsed_time(e1)})
     print(json.dumps({"profile_variants": out, "arenas": leg.n, "warmup_plain_decisions": 8}))
     del warm
     leg.free()
 
 
 def sweep(args, dev):
-    """The arena-count sweep (4,096 ... 1,048,576 arenas of one workload): the plain launch, the lockstep kernel and the
-    lockstep kernel with the learned binning (two bins, and sixteen cost levels), each timed on the same decisions from
-    the same start states; all words of the runs compared on the device, and a seeded 1% sample of the arenas replayed
-    through the oracle.  One JSON line per size."""
+    """The arena-count sweep (4,096 ... 1,048,576 arenas of one workload): the persistent kernel without barriers (one thread
+    per arena at every size, block 64), the plain call, the lockstep kernel and the lockstep kernel with the learned binning
+    (two bins, and sixteen cost levels), each timed on the same decisions from the same start states; all words of the runs
+    compared with the persistent kernel's on the device, and a seeded 1% sample of the arenas replayed through the oracle.
+    Every arm names the kernel that it ran; a ratio to the plain call is null where both ran the same launch.  One JSON
+    line per size."""
     import torch
     import rsx
     from runner import DecisionRunner
@@ -811,7 +806,8 @@ def sweep(args, dev):
         train_s = time.perf_counter() - t0
         base = {"block": 448, "grid": run.sms, "split": 15}
         out, words = {}, {}
-        for name, cfg in [("plain", {"mode": "plain", "block": 32}), ("lockstep", {"mode": "lockstep", **base}),
+        for name, cfg in [("persistent", {"mode": "persistent", "block": 64, "grid": run.sms * 8, "granularity": 1, "min_blocks": 8}),
+                          ("plain", {"mode": "plain", "block": 32}), ("lockstep", {"mode": "lockstep", **base}),
                           ("binned", {"mode": "binned", "threshold": 0.5, **base}),
                           ("levels", {"mode": "levels", "levels": 16, "weights": [1.0] * 6, **base})]:
             run.restore(start)
@@ -824,22 +820,22 @@ def sweep(args, dev):
             e1.record(run.stream)
             e1.synchronize()
             ms = e0.elapsed_time(e1) / D
-            out[name] = {"ms_per_decision": round(ms, 3), "arena_ticks_per_s": n * 8 / (ms / 1e3)}
+            out[name] = {"kernel": kernel_name(run, cfg), "ms_per_decision": round(ms, 3), "arena_ticks_per_s": n * 8 / (ms / 1e3)}
             words[name] = (run.snapshot(), run.res.clone())
-        exact = all(torch.equal(words[k][0], words["plain"][0]) and torch.equal(words[k][1], words["plain"][1]) for k in words)
+        exact = all(torch.equal(words[k][0], words["persistent"][0]) and torch.equal(words[k][1], words["persistent"][1]) for k in words)
+        plain_ms = out["plain"]["ms_per_decision"] if "lockstep" not in out["plain"]["kernel"] else None
+        vs = {f"{k}_vs_plain": plain_ms and plain_ms / out[k]["ms_per_decision"] for k in ("lockstep", "binned", "levels")}
         rec = {"arenas": n, "mix": args.mix, "decisions": D, "train_s": round(train_s, 2), **out,
-               "lockstep_vs_plain": out["plain"]["ms_per_decision"] / out["lockstep"]["ms_per_decision"],
-               "binned_vs_plain": out["plain"]["ms_per_decision"] / out["binned"]["ms_per_decision"],
-               "levels_vs_plain": out["plain"]["ms_per_decision"] / out["levels"]["ms_per_decision"],
+               **vs, "lockstep_vs_persistent": out["persistent"]["ms_per_decision"] / out["lockstep"]["ms_per_decision"],
                "bit_exact_all_arenas": bool(exact)}
         if L is not None and hasattr(L, "rsref_run_batch_ex"):
             rng = np.random.default_rng(args.seed + n)
             sample = np.sort(rng.choice(n, size=max(1, n // 100), replace=False))
-            # the plain run's final words and result words of the last decision; every decision's words through the oracle
+            # the persistent run's final words and result words of the last decision; every decision's words through the oracle
             a = torch.from_numpy(sample.astype(np.int64)).to(dev.device)[:, None]
             w = torch.arange(TICK_WORDS, device=dev.device, dtype=torch.int64)[None, :]
             pos = ((a // 32) * (32 * rsx.ARENA_WORDS) + w * 32 + (a % 32)).reshape(-1)
-            got = words["plain"][0][pos].reshape(len(sample), TICK_WORDS).cpu().numpy().view(np.uint32)
+            got = words["persistent"][0][pos].reshape(len(sample), TICK_WORDS).cpu().numpy().view(np.uint32)
             st0 = np.ascontiguousarray(st[sample])
             m = len(sample)
             res = np.zeros((D + 1, m), np.uint32)
@@ -850,7 +846,7 @@ def sweep(args, dev):
             smp = np.ascontiguousarray(sample.astype(np.uint32))
             L.rsref_run_batch_ex(st0.ctypes.data, m, sdsc.ctypes.data, sidx.ctypes.data, ctl_host.ctypes.data, n, smp.ctypes.data, D + 1, 0,
                                  res.ctypes.data, ev.ctypes.data)
-            last = words["plain"][1].index_select(0, a[:, 0]).cpu().numpy().view(np.uint32)
+            last = words["persistent"][1].index_select(0, a[:, 0]).cpu().numpy().view(np.uint32)
             rec["oracle_sample"] = {"arenas": m, "decisions": D + 1,
                                     "state_mismatches": int(np.any(st0[:, :TICK_WORDS] != got, axis=1).sum()),
                                     "last_result_mismatches": int((res[-1] != last).sum())}
@@ -926,7 +922,7 @@ def rollout_check(args, dev):
                 bad[d + 1] = int(np.any(got[d + 1] != ref[:, :TICK_WORDS], axis=1).sum())
         check = {"arenas": int(m), "at_decisions": checks, "mismatches": bad, "restarts_in_sample": resets,
                  "oracle_seconds": round(time.perf_counter() - t1, 1)}
-    print(json.dumps({"rollout": {"arenas": n, "decisions": D, "mix": "contact-heavy", "config": kernel_name(cfg) + " levels",
+    print(json.dumps({"rollout": {"arenas": n, "decisions": D, "mix": "contact-heavy", "config": kernel_name(run, cfg) + " levels",
                                   "initial_train_s": round(train_s, 2), "arena_ticks_per_s": n * 8 * D / (total_ms / 1e3),
                                   "windows": [{k: (round(v, 4) if isinstance(v, float) else v) for k, v in x.items()} for x in windows]},
                       "bit_exact_vs_oracle": check}))

@@ -89,9 +89,16 @@ int rsx_phase(rsx_device* dev, int k, rsx_states* st, rsx_static* sd, int32_t* d
 /* the copy-in / copy-out round trip (sim_identity[_tick], sim.cu:9-24) */
 int rsx_identity(rsx_device* dev, const uint32_t* d_in, uint32_t* d_out, uint32_t n, int tick_only);
 
-/* ---- extensions (no counterpart in the reference's kernel set; the functions above are unchanged by them) ----
+/* ---- extensions (no counterpart in the reference's kernel set; the functions above compute the same words without them,
+ * but rsx_sim8 launches the lockstep kernel below for a call of at most one arena per SM) ----
  * Per-arena car pairing: d_static points at `count` StaticData, sd_index[a] (u8, device memory) selects arena a's.  Up to
- * 256 arenas per SM the call runs the lockstep kernel below in a shape of the library's own (same words). */
+ * 256 arenas per SM the call runs the lockstep kernel below in a shape of the library's own (same words): its arenas are
+ * spread over every SM in blocks of 256 threads that leave no room for another.  By itself a call of played arenas is 1.6 -
+ * 3.6 times as fast as with one thread per arena (one of kickoffs, which hardly diverge, between 0.8 and 1.3 times), but
+ * calls on several streams run one after another: eight streams of 148 played arenas take 6.9 ms together and 6.0 with one
+ * thread per arena, of 1,024 each 14.4 and 7.3; of kickoffs 8.1 and 1.3, 9.6 and 1.6.  A program with many small batches
+ * in flight puts them into one call, or launches rsx_sim8_persistent_raw with a grid of n / 32 blocks of 32 threads, which
+ * is one thread per arena at any size. */
 int rsx_sim8_multi_raw(uint32_t* d_states, uint32_t n, const void* d_statics, const uint8_t* d_sd_index,
                        const rsx_controls* d_controls, uint32_t* d_result, uint32_t* d_event_or, uint32_t block, void* stream);
 /* The persistent kernel: `grid` resident blocks pull work items (32 x `granularity` arenas per warp) from a device
@@ -112,7 +119,7 @@ int rsx_sim8_persistent_ex(uint32_t* d_states, uint32_t n, const void* d_statics
                            uint32_t* d_cost, void* stream);
 /* The SM-lockstep persistent decision (no counterpart in the reference): `grid` resident blocks of `block` threads (a
  * multiple of 32, at most RSX_LOCKSTEP_MAX_BLOCK; normally one block per SM) step their warps' arenas phase by phase
- * together, so that all warps of an SM execute one phase's code at a time; each warp claims 32 entries of d_order
+ * together, so that all warps of an SM execute one phase's code at a time; each warp claims up to 32 entries of d_order
  * (identity when null) from d_queue_counter (cleared by the call) when its arenas finish.  split 1 adds a barrier after
  * each car's pre-tick inside P1; split 2 splits each car's P1 into pre-tick head, wheel rays and wheel response; split 3 adds a barrier
  * after every step of P3b's pair / leaf loop; split 4 / 5 drop the barriers from P3b / P4 to P8 (slower: kept for
@@ -124,10 +131,11 @@ int rsx_sim8_persistent_ex(uint32_t* d_states, uint32_t n, const void* d_statics
  * split 14 is split 11 with the 47 feature pairs of the box-triangle SATs that reach them computed by the whole block
  * (up to 18 SATs per round); split 15 runs a tick's mesh work in one round each for the wheel rays of both cars and for
  * every mesh pair of P3b, its BVH walks too by the whole block, level by level (the default: the fastest measured).  Split
- * 15 launches blocks no larger than their arenas need (256 or 384 threads, at 255 and 168 registers), and a call whose
- * arenas fit the grid in one round deals them out without the queue.  Register budget of the other sizes: 128.  Of a
- * grid past the device's SMs no more blocks are launched than it holds at once or than take the arenas.  At
- * most 2^24 arenas and grid 65,535 per call.  Results equal rsx_sim8_multi_raw's whatever grid, block, split or order. */
+ * 15 launches blocks no larger than their arenas need (256 or 384 threads, at 255 and 168 registers; the other sizes and
+ * splits have 128); a call of any split whose arenas fit the grid in one round deals them out without the queue
+ * (d_queue_counter is then not touched).  Of a grid past the device's SMs no more blocks are launched than it holds at once
+ * or than take the arenas.  At most 2^24 arenas and grid 65,535 per call.  Results equal rsx_sim8_multi_raw's whatever grid,
+ * block, split or order. */
 #define RSX_LOCKSTEP_MAX_BLOCK 512u
 int rsx_sim8_lockstep_raw(uint32_t* d_states, uint32_t n, const void* d_statics, const uint8_t* d_sd_index,
                           const rsx_controls* d_controls, uint32_t* d_result, uint32_t* d_event_or, const uint32_t* d_order,
@@ -142,6 +150,19 @@ int rsx_sim8_lockstep_ex(uint32_t* d_states, uint32_t n, const void* d_statics, 
                          const rsx_controls* d_controls, uint32_t* d_result, uint32_t* d_event_or, const uint32_t* d_order,
                          uint32_t* d_queue_counter, uint32_t grid, uint32_t block, uint32_t split, uint32_t ticks_per_launch,
                          void* stream);
+
+/* The launch that a decision of n arenas makes on the current device, for programs that name or compare launches: call
+ * RSX_CALL_SIM8 (rsx_sim8_raw without a trace) or RSX_CALL_MULTI (rsx_sim8_multi_raw) with the call's block (grid and split
+ * are not looked at), or RSX_CALL_LOCKSTEP with the grid, block and split of rsx_sim8_lockstep_raw.  Launches nothing. */
+#define RSX_CALL_SIM8 0
+#define RSX_CALL_MULTI 1
+#define RSX_CALL_LOCKSTEP 2
+typedef struct rsx_shape {
+  uint32_t lockstep;    /* 0: one thread per arena; else the block limit (256, 384, 448, 512) of the lockstep kernel's build */
+  uint32_t grid, block; /* blocks launched, threads of each */
+  uint32_t split, width, queue; /* lockstep: the barrier split, the arenas of a claim, 1 where claims come from the queue */
+} rsx_shape;
+int rsx_decision_shape(int call, uint32_t n, uint32_t grid, uint32_t block, uint32_t split, rsx_shape* out);
 
 /* The persistent decision without caller scratch (no counterpart in the reference): for callers that cannot allocate
  * device memory (their framework owns it, or cudaMalloc / cudaFree would synchronise a real-time loop), the work-queue

@@ -97,16 +97,17 @@ int rsx_set_last_error(int code, const char* msg) {
 // local memory (about 20 KB: the arena state and the solver's rows) by itself; nothing to configure per device.
 static int configure_current(void) { return RSX_OK; }
 
-// the lockstep kernel by register budget
+// the lockstep kernel by register budget (max_threads: its blocks' limit, which names the build)
 struct LockstepBuild {
+  uint32_t max_threads;
   decltype(&rsx_launch_sim8_lockstep_t448) launch;
   decltype(&rsx_lockstep_blocks_per_sm_t448) blocks_per_sm;
 };
 static LockstepBuild lockstep_build(uint32_t split, uint32_t block) {
-  if (split == kSpreadSplit && block <= 256) return {rsx_launch_sim8_lockstep_t256, rsx_lockstep_blocks_per_sm_t256};
-  if (split == kSpreadSplit && block <= 384) return {rsx_launch_sim8_lockstep_t384, rsx_lockstep_blocks_per_sm_t384};
-  if (block <= 448) return {rsx_launch_sim8_lockstep_t448, rsx_lockstep_blocks_per_sm_t448};
-  return {rsx_launch_sim8_lockstep_t512, rsx_lockstep_blocks_per_sm_t512};
+  if (split == kSpreadSplit && block <= 256) return {256, rsx_launch_sim8_lockstep_t256, rsx_lockstep_blocks_per_sm_t256};
+  if (split == kSpreadSplit && block <= 384) return {384, rsx_launch_sim8_lockstep_t384, rsx_lockstep_blocks_per_sm_t384};
+  if (block <= 448) return {448, rsx_launch_sim8_lockstep_t448, rsx_lockstep_blocks_per_sm_t448};
+  return {512, rsx_launch_sim8_lockstep_t512, rsx_lockstep_blocks_per_sm_t512};
 }
 static cudaError_t sm_count(uint32_t* sms) {
   int dev = 0, count = 0;
@@ -115,23 +116,34 @@ static cudaError_t sm_count(uint32_t* sms) {
   *sms = (uint32_t)count;
   return e;
 }
-// A decision in launches of ticks_per_launch ticks on up to `grid` blocks of up to `block` threads, on a device of `sms` SMs
-static cudaError_t lockstep(uint32_t* states, uint32_t n, const void* sds, const uint8_t* sd_index, const void* controls, uint32_t* result,
-                            uint32_t* ev_or, const uint32_t* order, uint32_t* counter, uint32_t grid, uint32_t block, uint32_t split,
-                            uint32_t ticks_per_launch, uint32_t sms, cudaStream_t s) {
+// The launch of a lockstep decision on up to `grid` blocks of up to `block` threads, on a device of `sms` SMs
+struct LockstepLaunch {
+  LockstepBuild build;
+  LockstepPlan plan;
+  uint32_t grid;
+};
+static cudaError_t lockstep_launch(uint32_t n, uint32_t grid, uint32_t block, uint32_t split, uint32_t sms, LockstepLaunch* l) {
   cudaError_t e = cudaSuccess;
-  grid = lockstep_grid(n, grid, block, sms, [&] {
+  l->grid = lockstep_grid(n, grid, block, sms, [&] {
     int blocks = 0;
     e = lockstep_build(split, block).blocks_per_sm((int)split, block, &blocks);
     return (uint32_t)blocks;
   });
-  const LockstepPlan p = lockstep_plan(n, grid, block, split);
+  l->plan = lockstep_plan(n, l->grid, block, split);
+  l->build = lockstep_build(split, l->plan.block);
+  return e;
+}
+// a decision in launches of ticks_per_launch ticks
+static cudaError_t lockstep(uint32_t* states, uint32_t n, const void* sds, const uint8_t* sd_index, const void* controls, uint32_t* result,
+                            uint32_t* ev_or, const uint32_t* order, uint32_t* counter, uint32_t grid, uint32_t block, uint32_t split,
+                            uint32_t ticks_per_launch, uint32_t sms, cudaStream_t s) {
+  LockstepLaunch l;
+  cudaError_t e = lockstep_launch(n, grid, block, split, sms, &l);
   for (uint32_t t0 = 1; t0 <= RSX_TICKS_PER_DECISION && e == cudaSuccess; t0 += ticks_per_launch) {
-    if (p.queue) e = cudaMemsetAsync(counter, 0, 4, s);
+    if (l.plan.queue) e = cudaMemsetAsync(counter, 0, 4, s);
     if (e == cudaSuccess)
-      e = lockstep_build(split, p.block)
-              .launch(states, sds, sd_index, controls, result, ev_or, order, p.queue ? counter : nullptr, n, p.width, grid, p.block, (int)split,
-                      t0, t0 + ticks_per_launch - 1, s);
+      e = l.build.launch(states, sds, sd_index, controls, result, ev_or, order, l.plan.queue ? counter : nullptr, n, l.plan.width, l.grid,
+                         l.plan.block, (int)split, t0, t0 + ticks_per_launch - 1, s);
   }
   return e;
 }
@@ -144,9 +156,10 @@ static cudaError_t lockstep(uint32_t* states, uint32_t n, const void* sds, const
 //     per SM (37 arenas: 1.2 ms, 1.7 - 2.5 in warps of 32; 148: 1.2 and 3.0, kickoffs 0.89 and 0.98): from there on kickoffs
 //     of one pairing, which neither diverge nor read different StaticData, are faster in few full warps (1,024: 1.00 ms,
 //     1.15 in the lockstep kernel).
-//   above: one thread per arena in the caller's blocks, the reference's shape, which the lockstep kernel's timings at those
-//     sizes are compared with.
+//   above: one thread per arena in the caller's blocks, the reference's shape (rsx_sim8_lockstep_raw is the faster call for
+//     such batches, but for a small one of kickoffs: 37,889 arenas through rsx_sim8_multi_raw take 25 ms, 37,888 7.9).
 enum class Shape { kLanes, kLockstep, kPlain };
+constexpr uint32_t kSim8PerSm = 1, kMultiPerSm = kSpreadBlock;  // `most`
 static cudaError_t one_launch_shape(uint32_t n, uint32_t most_per_sm, uint32_t* sms, Shape* shape) {
   const cudaError_t e = sm_count(sms);
   *shape = n <= *sms / 8 ? Shape::kLanes : n <= *sms * most_per_sm ? Shape::kLockstep : Shape::kPlain;
@@ -262,7 +275,7 @@ int rsx_sim8_raw(uint32_t* d_states, uint32_t n, const void* d_static, const rsx
   if (c != RSX_OK) return c;
   uint32_t sms = 0;
   Shape shape = Shape::kPlain;
-  if (!d_trace) RSX_CK(one_launch_shape(n, 1, &sms, &shape));
+  if (!d_trace) RSX_CK(one_launch_shape(n, kSim8PerSm, &sms, &shape));
   if (shape == Shape::kLockstep)
     RSX_CK(lockstep(d_states, n, d_static, nullptr, d_controls, d_result, nullptr, nullptr, nullptr, sms, kSpreadBlock, kSpreadSplit,
                     RSX_TICKS_PER_DECISION, sms, (cudaStream_t)stream));
@@ -304,7 +317,7 @@ int rsx_sim8_multi_raw(uint32_t* d_states, uint32_t n, const void* d_statics, co
   if (c != RSX_OK) return c;
   uint32_t sms = 0;
   Shape shape = Shape::kPlain;
-  RSX_CK(one_launch_shape(n, kSpreadBlock, &sms, &shape));
+  RSX_CK(one_launch_shape(n, kMultiPerSm, &sms, &shape));
   if (shape == Shape::kLockstep)
     RSX_CK(lockstep(d_states, n, d_statics, d_sd_index, d_controls, d_result, d_event_or, nullptr, nullptr, sms, kSpreadBlock,
                     kSpreadSplit, RSX_TICKS_PER_DECISION, sms, (cudaStream_t)stream));
@@ -376,6 +389,27 @@ int rsx_sim8_lockstep_ex(uint32_t* d_states, uint32_t n, const void* d_statics, 
   RSX_CK(sm_count(&sms));
   RSX_CK(lockstep(d_states, n, d_statics, d_sd_index, d_controls, d_result, d_event_or, d_order, d_queue_counter, grid, block, split,
                   ticks_per_launch, sms, (cudaStream_t)stream));
+  return RSX_OK;
+}
+
+int rsx_decision_shape(int call, uint32_t n, uint32_t grid, uint32_t block, uint32_t split, rsx_shape* out) {
+  const bool queue_call = call == RSX_CALL_LOCKSTEP;
+  if (!out || n == 0 || call < RSX_CALL_SIM8 || call > RSX_CALL_LOCKSTEP || block == 0 || (queue_call && grid == 0)) return RSX_E_ARG;
+  uint32_t sms = 0;
+  Shape shape = Shape::kLockstep;
+  if (queue_call)
+    RSX_CK(sm_count(&sms));
+  else
+    RSX_CK(one_launch_shape(n, call == RSX_CALL_SIM8 ? kSim8PerSm : kMultiPerSm, &sms, &shape));
+  if (shape != Shape::kLockstep) {
+    const uint32_t b = shape == Shape::kLanes ? 1 : block;
+    *out = {0, (n + b - 1) / b, b, 0, 0, 0};
+    return RSX_OK;
+  }
+  LockstepLaunch l;
+  if (!queue_call) split = kSpreadSplit;
+  RSX_CK(lockstep_launch(n, queue_call ? grid : sms, queue_call ? block : kSpreadBlock, split, sms, &l));
+  *out = {l.build.max_threads, l.grid, l.plan.block, split, l.plan.width, l.plan.queue ? 1u : 0u};
   return RSX_OK;
 }
 

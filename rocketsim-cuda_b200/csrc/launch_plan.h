@@ -34,10 +34,11 @@ inline LockstepPlan lockstep_plan(uint32_t n, uint32_t grid, uint32_t block, uin
   const uint64_t rounds = (n + lanes - 1) / lanes;
   const uint32_t per = (uint32_t)((n + rounds * grid - 1) / (rounds * grid));  // a block's arenas in one round
   LockstepPlan p;
-  // Blocks no larger than their arenas need: a scheduler's registers are its warps', and the simulator's inlined phases
-  // spill less in 255 registers (8 warps) or 168 (12) than in 128 (14 and 16).  20,000 arenas (136 per SM): 6.4 ms in 256
-  // threads, 7.5 in 448; 56,000 (379): 10.6 in 384, 11.2 in 448.  Uneven rounds are evened out the same way: 70,001
-  // arenas in two rounds of 256 threads rather than one of 448 and a rest.
+  // Blocks no larger than their arenas need: a scheduler's registers are its warps', 255 each for 8 warps a block, 168 for 12,
+  // 128 for 14 and 16.  20,000 headline arenas (136 per SM): 6.5 ms in 256 threads; 7.3 in 448, and 7.8 in 256 threads held
+  // to 128 registers, so it is the registers that pay and not the fewer warps at a barrier.  56,000 (379): 9.7 in 384, 10.1
+  // in 448.  Uneven rounds are evened out the same way: 70,001 arenas in two rounds of 256 threads rather than one of 448
+  // and a rest.
   p.block = block;
   if (split == kSpreadSplit && per <= 384 && block > 384) p.block = 384;
   if (split == kSpreadSplit && per <= 256 && block > 256) p.block = 256;

@@ -100,6 +100,7 @@ def lib() -> ctypes.CDLL:
                                             ctypes.c_uint32, vp]
         L.rsx_sim8_lockstep_ex.argtypes = [vp, ctypes.c_uint32, vp, vp, vp, vp, vp, vp, vp, ctypes.c_uint32, ctypes.c_uint32,
                                            ctypes.c_uint32, ctypes.c_uint32, vp]
+        L.rsx_decision_shape.argtypes = [ctypes.c_int, ctypes.c_uint32, ctypes.c_uint32, ctypes.c_uint32, ctypes.c_uint32, vp]
         L.rsx_copy_raw.argtypes = [vp, vp, ctypes.c_uint64, vp]
         L.rsx_make_states_at.argtypes = [u32p, ctypes.c_uint32, vp, vp, ctypes.c_uint32, ctypes.c_uint64, ctypes.POINTER(ctypes.c_float), u32p]
         L.rsx_l2_persist_raw.argtypes = [vp, ctypes.c_uint64, ctypes.c_float, vp]
@@ -118,6 +119,17 @@ def lib() -> ctypes.CDLL:
         L.rsx_v3_write_arena.argtypes = [u32p, u32p, tp, vp, ctypes.c_size_t, szp]
         _lib = L
     return _lib
+
+
+CALL_SIM8, CALL_MULTI, CALL_LOCKSTEP = 0, 1, 2  # the call of decision_shape
+
+
+def decision_shape(call: int, n: int, block: int, grid: int = 0, split: int = 0) -> dict:
+    """The launch that a decision of n arenas makes on the current device (rsx_decision_shape)."""
+    names = ("lockstep", "grid", "block", "split", "width", "queue")
+    out = (ctypes.c_uint32 * len(names))()
+    check(lib().rsx_decision_shape(call, n, grid, block, split, out), "rsx_decision_shape")
+    return dict(zip(names, out))
 
 
 class V3Template(ctypes.Structure):

@@ -4,8 +4,10 @@ decisions, and the autotuner that picks the launch configuration.
 A `DecisionRunner` owns the device buffers of one batch of arenas (AoSoA-32 states, per-arena car pairing, results,
 event words, queue counter, arena order, predictor features and logits) and issues one decision with `step()`:
 
-  sim8        k_sim8 through rsx_sim8_raw: the reference's sim8 entry (one StaticData for all arenas, block 32)
-  plain       k_sim8_multi, one thread per arena, one launch per decision (the reference's sim8 shape, block 32)
+  sim8        rsx_sim8_raw: the reference's sim8 entry (one StaticData for all arenas, block 32); one thread per arena
+              (k_sim8) above one arena per SM, the lockstep kernel or one lane per SM up to there
+  plain       rsx_sim8_multi_raw, one launch per decision: one thread per arena (k_sim8_multi, the reference's sim8 shape,
+              block 32) above 256 arenas per SM, the lockstep kernel or one lane per SM up to there
   persistent  the persistent kernel without barriers (rsx_sim8_persistent_ex): register budget and queue granularity
   lockstep    the SM-lockstep persistent kernel (rsx_sim8_lockstep_ex) over the identity order, 8 / `ticks` launches
               of `ticks` ticks per decision (default 8: one launch)
@@ -112,6 +114,27 @@ class DecisionRunner:
                                          self.ev.data_ptr(), order, self.counter.data_ptr(), c.get("grid", self.sms), c["block"],
                                          c["split"], c.get("ticks", 8), self.sptr), "rsx_sim8_lockstep_ex")
 
+    def launch(self, config: dict | None = None) -> tuple:
+        """What identifies a configuration's decision launches at this size: the kernel and its shape (rsx.decision_shape).
+        Configurations with the same launch and order are one."""
+        c = config or self.config
+        if c["mode"] == "persistent":
+            return ("persistent", c["min_blocks"], c["grid"], c["block"], c["granularity"])
+        with self.torch.cuda.device(self.dev.device):
+            if c["mode"] in ("sim8", "plain"):
+                call = rsx.CALL_SIM8 if c["mode"] == "sim8" else rsx.CALL_MULTI
+                s = rsx.decision_shape(call, self.n, c.get("block", 32))
+            else:
+                s = rsx.decision_shape(rsx.CALL_LOCKSTEP, self.n, c["block"], c.get("grid", self.sms), c["split"])
+        if not s["lockstep"]:
+            return ("k_sim8" if c["mode"] == "sim8" else "k_sim8_multi", s["grid"], s["block"])
+        return (f"k_sim8_lockstep_t{s['lockstep']}<{s['split']}>", s["grid"], s["block"], s["width"], s["queue"], c.get("ticks", 8))
+
+    def kernel(self, config: dict | None = None) -> str:
+        """The name of the kernel that a configuration's decision runs at this size."""
+        c = config or self.config
+        return f"k_sim8_persistent_b{c['min_blocks']}" if c["mode"] == "persistent" else self.launch(c)[0]
+
     def kernels_per_step(self, config: dict | None = None) -> int:
         """This library's kernel launches per decision (features, forward, two binning passes or three level passes,
         and the decision's launches: 8 / ticks per launch for the lockstep kernel)."""
@@ -171,13 +194,14 @@ class DecisionRunner:
 
     # ---- the autotuner ----
     def candidates(self, binning: bool = True):
-        # the plain launch too: with few arenas per SM (a few thousand arenas) the barriers cost more than they save
+        # one thread per arena (at sizes where rsx_sim8_multi_raw runs the lockstep kernel, that kernel's launch)
         out = [{"mode": "plain", "block": 32}, {"mode": "plain", "block": 64}]
         # the persistent kernel without barriers: register budget (min_blocks of 64 threads per SM) and queue granularity
         for min_blocks, gran in ((8, 1), (8, 4), (12, 1)):
             out.append({"mode": "persistent", "block": 64, "grid": self.sms * min_blocks, "granularity": gran, "min_blocks": min_blocks})
         # splits: 7 (lockstep), 14 (+ P3b's mesh-leaf tests, the SATs' feature pairs and the wheel rays' mesh leaves
-        # pooled over the block, P3a in one piece), 15 (14 with the wheel rays' mesh walks pooled too)
+        # pooled over the block, P3a in one piece), 15 (a tick's mesh work in one round each for both cars' wheel rays and
+        # for P3b, the walks by the whole block too)
         for block, split in itertools.product((448, 512), (7, 14, 15)):
             out.append({"mode": "lockstep", "block": block, "grid": self.sms, "split": split, "threshold": None})
             if split == 15:  # ticks per launch: a decision in 2 or 4 launches, arenas re-claimed (re-balanced) between them
@@ -188,7 +212,15 @@ class DecisionRunner:
                     out.append({"mode": "binned", "block": block, "grid": self.sms, "split": split, "threshold": thr, "labels": labels})
                 out.append({"mode": "levels", "block": block, "grid": self.sms, "split": split, "threshold": None, "levels": 16,
                             "weights": [1.0] * P.LABELS})
-        return out
+        # with few arenas a block, blocks of 448 and of 512 (and the plain call) are one and the same launch
+        seen, different = set(), []
+        for c in out:
+            order = (c["mode"], c["threshold"], c.get("labels")) if c["mode"] in ("binned", "levels") else None
+            key = (self.launch(c), order)
+            if key not in seen:
+                seen.add(key)
+                different.append(c)
+        return different
 
     def tune(self, controls_ptrs, candidates=None, repeats: int = 1, margin: float = 0.01):
         """Times every candidate on the same decisions from the same start states, `repeats` times each (the candidates

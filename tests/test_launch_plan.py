@@ -121,11 +121,12 @@ def test_lockstep_blocks(rsx, dev, n, grid, block):
 
 
 def test_rounds_and_plain_at_size(rsx, dev):
-    """Two even rounds of the smaller budget, and the plain launch above the lockstep kernel's sizes."""
+    """Two even rounds of the smaller budget, and the plain launch above the lockstep kernel's sizes, block 32 and 64."""
     n = SMS * 448 + 77
     a = Arenas(rsx, dev, n)
     a.same(a.lockstep)
     a.same(a.multi)
+    a.same(lambda: a.multi(64))
     a.free()
 
 

@@ -1,6 +1,7 @@
-"""The batching layer (runner.DecisionRunner): the plain launch, the lockstep kernel launched one by one and as a CUDA
-graph, and the learned-binning order give the same words after several decisions, and the autotuner leaves the states
-as it found them (it times candidates on a snapshot)."""
+"""The batching layer (runner.DecisionRunner): the plain call, the lockstep kernel launched one by one and as a CUDA graph,
+the learned-binning order and the persistent kernel without barriers (one thread per arena at every size) give the same
+words after several decisions, the autotuner leaves the states as it found them (it times candidates on a snapshot), and
+its candidates are different launches."""
 import numpy as np
 import pytest
 
@@ -26,6 +27,7 @@ def test_modes_graphs_and_autotuner_agree(rsx):
         modes = [{"mode": "plain", "block": 32},
                    {"mode": "lockstep", "block": 448, "grid": run.sms, "split": 1},
                    {"mode": "lockstep", "block": 64, "grid": 3, "split": 0},
+                   {"mode": "persistent", "block": 64, "grid": run.sms * 4, "granularity": 1, "min_blocks": 8},
                    {"mode": "binned", "block": 384, "grid": run.sms, "split": 1, "threshold": 0.3}]
         outs = []
         for i, c in enumerate(modes):
@@ -56,3 +58,37 @@ def test_modes_graphs_and_autotuner_agree(rsx):
         run.free()
     finally:
         dev.close()
+
+
+def test_launches_are_named_and_candidates_differ(rsx):
+    """A configuration's launch at the sizes where it changes, and no two tuner candidates of one launch and order."""
+    from runner import DecisionRunner
+
+    dev = rsx.SimDevice(0)
+    try:
+        sds = rsx.build_static(7, 0, 0)[None]
+        sms = dev.torch.cuda.get_device_properties(dev.device).multi_processor_count
+        plain = [{"mode": "plain", "block": b} for b in (32, 64)]
+        lock = [{"mode": "lockstep", "block": b, "grid": sms, "split": 15} for b in (448, 512)]
+        for n, names, same_plain, same_lock in ((sms // 8, ("k_sim8_multi", "k_sim8_lockstep_t256<15>"), True, True),
+                                                (256 * sms, ("k_sim8_lockstep_t256<15>", "k_sim8_lockstep_t256<15>"), True, True),
+                                                (256 * sms + 1, ("k_sim8_multi", "k_sim8_lockstep_t384<15>"), False, True),
+                                                (384 * sms + 1, ("k_sim8_multi", "k_sim8_lockstep_t448<15>"), False, False)):
+            run = DecisionRunner(_Allocated(dev), sds, np.zeros(n, np.uint8), np.broadcast_to(np.zeros(1, np.uint32), (n, 1)))
+            assert (run.kernel(plain[0]), run.kernel(lock[0])) == names, n
+            assert (run.launch(plain[0]) == run.launch(plain[1])) == same_plain and (run.launch(lock[0]) == run.launch(lock[1])) == same_lock, n
+            cands = run.candidates(binning=False)
+            assert len({run.launch(c) for c in cands}) == len(cands), n
+            run.free()
+        assert rsx.lib().rsx_decision_shape(rsx.CALL_MULTI, 0, 0, 32, 0, None) == -1
+    finally:
+        dev.close()
+
+
+class _Allocated:
+    """A device whose uploaded states are only allocated (nothing here steps them)."""
+
+    def __init__(self, dev):
+        self.__dict__.update(dev.__dict__)
+        self.upload_static = dev.upload_static
+        self.upload_states = lambda states: dev.alloc_states(states.shape[0])
