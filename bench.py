@@ -63,13 +63,13 @@ def _kc(rd, wr, inst, thr):
 
 
 KERNEL_COUNTERS = {
-    "k_sim8_multi": _kc(5058114816, 5021709056, 1509326896, 9997320896),
-    "k_sim8_lockstep_t448<7>": _kc(6146897920, 5795379200, 1581091634, 10610346282),
-    "k_sim8_lockstep_t512<7>": _kc(6137490176, 5792792832, 1581875941, 10635629271),
-    "k_sim8_lockstep_t448<14>": _kc(5886416640, 5595306496, 1189371246, 11172830549),
-    "k_sim8_lockstep_t512<14>": _kc(5900027648, 5608007168, 1192384700, 11263047794),
-    "k_sim8_lockstep_t448<15>": _kc(5450868736, 5343553280, 990985466, 11269310229),
-    "k_sim8_lockstep_t512<15>": _kc(5474784256, 5368506112, 992948195, 11330182713),
+    "k_sim8_multi": _kc(5012664832, 4983213056, 1509326896, 9997320896),
+    "k_sim8_lockstep_t448<7>": _kc(6170917376, 5804142592, 1526494951, 10299565331),
+    "k_sim8_lockstep_t512<7>": _kc(6174076160, 5801423616, 1527099371, 10318948146),
+    "k_sim8_lockstep_t448<14>": _kc(5866943744, 5585622272, 1184789126, 11036995067),
+    "k_sim8_lockstep_t512<14>": _kc(5885379840, 5596246528, 1187497356, 11124560523),
+    "k_sim8_lockstep_t448<15>": _kc(5453362176, 5341567488, 990819667, 11266854962),
+    "k_sim8_lockstep_t512<15>": _kc(5474244096, 5365953536, 992951527, 11326782781),
 }
 
 

@@ -90,7 +90,7 @@ def test_sim8_matches_oracle(rsx, dev, idx):
 
 
 def test_result_independent_of_block_order_and_queue(rsx, dev):
-    """Block 32 vs 64, the multi-static kernel, the persistent kernel over a permuted order with several queue
+    """Block 32 vs 64, the multi-static call (at this size a lockstep launch), the persistent kernel over a permuted order with several queue
     granularities, and the SM-lockstep kernel over several grids, blocks, barrier splits and orders (grid 2 x 64
     threads: 4 warps take 32 claims in turn) give the same words (the reference's determinism test,
     tests/step.rs:455-506)."""

@@ -1,7 +1,7 @@
 """The orders in which the lockstep kernel's split 15 runs a tick's pieces, arena by arena on the host build, against the
 phases they replace, word for word on contact-rich play with demolitions and respawns: both cars' wheel rays before car
-0's response (P1), the sorts of P3a over the axes that have an edge to pass against one loop per end and direction, and
-P3b with its mesh jobs found, walked level by level and tested before any pair runs."""
+0's response (P1), and P3b with its mesh jobs found, walked level by level and tested before any pair runs.  On the same
+play P3a's sort, which every split shares, against its rule restated one step at a time (one loop per end and direction)."""
 import os
 import shutil
 import subprocess
