@@ -23,7 +23,7 @@
 // than a warp leaves its other lanes without an arena; they still take part in the block's pooled work.  A decision split
 // over several launches carries each arena's progress in its result word (scored tick, unimplemented bit) and event
 // word; an arena scored in an earlier launch is not stepped again.  The block leaves when no warp holds work.  Lanes past
-// n (and order entries past n) step nothing.
+// n and order entries past n store nothing (they step nothing, or a copy in the splits that pool nothing).
 //
 // Results: each arena's decision is the decide() sequence of sim/physics.cuh (controls before every tick, all 8 ticks
 // stepped, the state after the first scored tick kept, event OR up to that tick), so states, result words and event

@@ -74,9 +74,9 @@ class Arenas:
         self.rsx.check(self.L.rsx_sim8_raw(self.ds.ptr(), self.n, self.sd.ptr(), self.ctl.data_ptr(), self.res.data_ptr(), 32, None,
                                            self.dev.stream_ptr()), "sim8")
 
-    def lockstep(self, grid=SMS, block=448, order=None, ticks=8):
+    def lockstep(self, grid=SMS, block=448, order=None, ticks=8, split=15):
         self.rsx.check(self.L.rsx_sim8_lockstep_ex(self.ds.ptr(), self.n, self.sd.ptr(), self.idx.data_ptr(), self.ctl.data_ptr(),
-                                                   self.res.data_ptr(), self.ev.data_ptr(), order, self.counter.data_ptr(), grid, block, 15,
+                                                   self.res.data_ptr(), self.ev.data_ptr(), order, self.counter.data_ptr(), grid, block, split,
                                                    ticks, self.dev.stream_ptr()), "lockstep")
 
     def free(self):
@@ -127,6 +127,48 @@ def test_rounds_and_plain_at_size(rsx, dev):
     a.same(a.lockstep)
     a.same(a.multi)
     a.same(lambda: a.multi(64))
+    a.free()
+
+
+# an order that leaves arenas out (entries of n or more step nothing): some of a claim, the whole of another; lanes past the
+# arenas step copies below split 9 and nothing from there
+@pytest.mark.parametrize("split", [0, 1, 7, 9, 14, 15])
+@pytest.mark.parametrize("grid,block,ticks", [(2, 64, 8), (148, 448, 4)])
+def test_orders_with_holes(rsx, dev, split, grid, block, ticks):
+    n = 203
+    a = Arenas(rsx, dev, n)
+    rng = np.random.default_rng(8)
+    order = rng.permutation(n).astype(np.int32)
+    holes = np.r_[5:9, 64:128, n - 2]  # positions 64 .. 127 hold a whole claim of the wide launches
+    left_out = np.sort(order[holes])
+    order[holes] = n + np.arange(len(holes), dtype=np.int32)
+    d_order = a.t.from_numpy(order).to(dev.device)
+    got = a.step(lambda: a.lockstep(grid, block, d_order.data_ptr(), ticks, split))
+    kept = np.ones(n, bool)
+    kept[left_out] = False
+    for g, w, name in zip(got[1:], a.want[1:], ("results", "events")):
+        g, w = g.cpu().numpy(), w.cpu().numpy()
+        assert np.array_equal(g[kept], w[kept]) and (g[~kept] == -1).all(), name
+    states, want, start = (rsx.unpack(x.cpu().numpy().view(np.uint32), n) for x in (got[0], a.want[0], a.start))
+    assert np.array_equal(states[kept][:, :rsx.TICK_WORDS], want[kept][:, :rsx.TICK_WORDS])
+    assert np.array_equal(states[~kept], start[~kept])
+    a.free()
+
+
+def test_a_first_launch_inside_a_capture(rsx, dev):
+    """A grid past the SMs (whose blocks the library counts first) and a small one-launch decision, captured and replayed."""
+    a = Arenas(rsx, dev, 4096)
+    for f in (lambda: a.lockstep(1480, 96), a.multi):
+        s = a.t.cuda.ExternalStream(dev.stream_ptr(), device=dev.device)
+
+        def captured():
+            g = a.t.cuda.CUDAGraph()
+            with a.t.cuda.graph(g, stream=s):
+                f()
+            with a.t.cuda.stream(s):
+                g.replay()
+
+        a.same(captured)
     a.free()
 
 

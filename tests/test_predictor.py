@@ -202,6 +202,60 @@ def test_forward_and_gradients_match_reference():
     assert abs(float(pr.loss.item()) / n - loss_ref) < 2e-2 * abs(loss_ref)
 
 
+def batch(n, seed):
+    """n feature rows (BF16 values, and their words on the device) and label bytes."""
+    import torch
+
+    dev = torch.device("cuda", 0)
+    rng = np.random.default_rng(seed)
+    X = bf16(rng.normal(0, 1, (n, 48)).astype(np.float32))
+    Y = rng.integers(0, 64, n).astype(np.uint8)
+    return X, torch.from_numpy((X.view(np.uint32) >> 16).astype(np.uint16).view(np.int16)).to(dev), Y, torch.from_numpy(Y).to(dev)
+
+
+# the weight gradients take 128 rows a CTA up to 2,048 and 256 above, in chunks of 64: one row, the edges of a chunk, of a slice
+# and of the rule, a last slice of one row
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [1, 63, 65, 128, 129, 2047, 2048, 2049, 2305])
+def test_gradients_at_the_slices_edges(n):
+    import torch
+
+    X, Xw, Y, Yd = batch(n, n)
+    pr = P.ContactPredictor(torch.device("cuda", 0), seed=2)
+    p = pr.params()
+    pr.gradients(Xw, Yd, n)
+    torch.cuda.synchronize()
+    _, g_ref, _ = reference(p, X, Y)
+    g = P.unpack_params(pr.grad.cpu().numpy())
+    for k, ref in g_ref.items():
+        assert rel(g[k], ref) < 2e-2, f"gradient {k}: relative difference {rel(g[k], ref):.4f}"
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("off", [1, 2, 4])
+def test_weights_off_a_16_byte_boundary(off):
+    """The BF16 weights `off` elements past a 16-byte boundary are staged value by value: the same operands, so the same bits
+    of the logits; the gradients' FP32 sums have up to 100 terms whose order is not fixed (100 x 2^-24 = 6e-6)."""
+    import torch
+
+    n = 100
+    _, Xw, _, Yd = batch(n, 3)
+    pr = P.ContactPredictor(torch.device("cuda", 0), seed=2)
+    z = pr.logits(Xw, n).clone()
+    g = pr.gradients(Xw, Yd, n).clone()
+    moved = torch.empty(pr.wb.numel() + 8, dtype=pr.wb.dtype, device=pr.wb.device)[off:off + pr.wb.numel()]
+    moved.copy_(pr.wb)
+    assert pr.wb.data_ptr() % 16 == 0 and moved.data_ptr() % 16 == 2 * off
+    torch.cuda.synchronize()
+    pr.wb = moved
+    z2 = pr.logits(Xw, n)
+    g2 = pr.gradients(Xw, Yd, n)
+    torch.cuda.synchronize()
+    assert int(pr.tc_error.item()) == 0
+    assert torch.equal(z[:, :6], z2[:, :6])
+    assert rel(g2.cpu().numpy(), g.cpu().numpy()) < 6e-6
+
+
 @pytest.mark.gpu
 def test_training_lowers_loss_and_binning_orders_heavy_first():
     import torch
